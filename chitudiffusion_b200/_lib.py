@@ -40,6 +40,8 @@ EXPORTS = (
     "chitu_b200_peer_wait_outputs",
     "chitu_b200_attn_splitkv_workspace_bytes",
     "chitu_b200_attn_fwd_splitkv",
+    "chitu_b200_attn_balanced_workspace_bytes",
+    "chitu_b200_attn_fwd_balanced",
     "chitu_b200_attn_fwd_splitkv_static",
     "chitu_b200_qk_norm_rope_batch",
     "chitu_b200_layernorm_modulate",
@@ -155,6 +157,14 @@ def load() -> ctypes.CDLL:
         _vp, _vp, _vp, _vp, _vp,
         ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
         _i64p, _i64p, _i64p, ctypes.c_float, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int64, _vp, _vp,
+    ]
+    lib.chitu_b200_attn_balanced_workspace_bytes.restype = ctypes.c_int64
+    lib.chitu_b200_attn_balanced_workspace_bytes.argtypes = [ctypes.c_int] * 4
+    lib.chitu_b200_attn_fwd_balanced.restype = ctypes.c_int
+    lib.chitu_b200_attn_fwd_balanced.argtypes = [
+        _vp, _vp, _vp, _vp, _vp,
+        ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+        _i64p, _i64p, _i64p, ctypes.c_float, ctypes.c_int, _vp, ctypes.c_int64, _vp, _vp,
     ]
     lib.chitu_b200_attn_fwd_splitkv_static.restype = ctypes.c_int
     lib.chitu_b200_attn_fwd_splitkv_static.argtypes = [

@@ -164,6 +164,102 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
   return r;
 }
 
+// One softmax step of a query tile's four warps (thread = one row, 128 scores): scores in, probabilities out.
+//
+//   t_s / t_o   this warp's tensor-memory addresses of the tile's scores and accumulator
+//   bar_p       the tile's two hand-over barriers (keys [0, 64) and [64, 128); every thread arrives)
+//   first       no accumulator yet
+//   valid       keys of this tile that exist (kTileN: all)
+template <bool kFp16>
+__device__ __forceinline__ void softmax_step(uint32_t t_s, uint32_t t_o, uint32_t bar_p, bool first, int valid, float sl2,
+                                             float& m_used, float& l_sum) {
+  // Row of 128 scores into registers, 32 columns per load; the load of chunk
+  // c+1 is in flight while the running maximum of chunk c is taken.
+  uint32_t s[4][32];
+  float mx0 = -INFINITY, mx1 = -INFINITY;
+  tmem_ld32(t_s, s[0]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    tmem_wait_ld();
+    if (c < 3) tmem_ld32(t_s + (c + 1) * 32, s[c + 1]);
+    if (valid < kTileN) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (c * 32 + i >= valid) s[c][i] = 0xff800000u;  // -inf
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      mx0 = max3(mx0, __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+      mx1 = max3(mx1, __uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3]));
+    }
+  }
+  const float mx = fmaxf(mx0, mx1);
+
+  if (first) {
+    m_used = mx;
+  } else {
+    const bool need = (mx - m_used) * sl2 > kRescaleThreshold;
+    if (__any_sync(0xffffffffu, need)) {
+      const float f = need ? fast_exp2((m_used - mx) * sl2) : 1.0f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t o[32];
+        tmem_ld32(t_o + c * 32, o);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+        tmem_st32(t_o + c * 32, o);
+      }
+      l_sum *= f;
+      if (need) m_used = mx;
+    }
+  }
+
+  // p = 2^(s*scale - m*scale): packed two-wide FMA / add, one MUFU per element
+  const float2 sl2_2 = make_float2(sl2, sl2);
+  // (a row without a finite score so far has nothing to subtract: its probabilities are zero, not NaN)
+  const float neg_m = m_used == -INFINITY ? 0.f : -m_used * sl2;
+  const float2 neg_m2 = make_float2(neg_m, neg_m);
+  uint32_t pk[2][32];
+  float2 la = make_float2(0.f, 0.f), lb = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      float2 x0 = __ffma2_rn(make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sl2_2, neg_m2);
+      float2 x1 =
+          __ffma2_rn(make_float2(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3])), sl2_2, neg_m2);
+      // kPolyPairs of every 8 pairs take the FMA-pipe polynomial, the rest the MUFU unit, so
+      // that both pipes stay busy (this iteration handles pairs 2g and 2g+1, g = i / 4)
+      constexpr int kPolyOdd = kPolyPairs < 4 ? kPolyPairs : 4;
+      constexpr int kPolyEven = kPolyPairs > 4 ? kPolyPairs - 4 : 0;
+      if (((i >> 2) & 3) < kPolyEven) {
+        x0 = exp2_poly2(x0);
+      } else {
+        x0.x = fast_exp2(x0.x);
+        x0.y = fast_exp2(x0.y);
+      }
+      if (((i >> 2) & 3) < kPolyOdd) {
+        x1 = exp2_poly2(x1);
+      } else {
+        x1.x = fast_exp2(x1.x);
+        x1.y = fast_exp2(x1.y);
+      }
+      la = __fadd2_rn(la, x0);
+      lb = __fadd2_rn(lb, x1);
+      pk[c >> 1][(c & 1) * 16 + (i >> 1)] = pack2<kFp16>(x0.x, x0.y);
+      pk[c >> 1][(c & 1) * 16 + (i >> 1) + 1] = pack2<kFp16>(x1.x, x1.y);
+      if ((c & 1) == 1 && i == 28) {
+        // 64 probabilities done: hand this half to the MMA warp
+        tmem_st32(t_s + (c >> 1) * 32, pk[c >> 1]);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(bar_p + 8 * (c >> 1));
+      }
+    }
+  l_sum += (la.x + la.y) + (lb.x + lb.y);
+}
+
 // The four softmax warps of a query tile rewrite it in shared memory.  As in the pre-pass kernel a
 // thread owns one 8-value vector (16 threads per row, so a warp works on two rows at a time and the
 // tile takes 16 rounds); the sum of squares is the same 16-lane butterfly, so the numbers match the
@@ -723,117 +819,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       float m_used = -INFINITY;
       float l_sum = 0.f;
 
-#ifdef CHITU_ATTN_TIMING
-      long long tw = 0, tl = 0, tm = 0, ts = 0, c0, c1;
-#define TICK(acc) c1 = clock64(); acc += c1 - c0; c0 = c1;
-#else
-#define TICK(acc)
-#endif
       int jt = rot;  // the CTA's tile of step j (advanced without a division)
       // the tile whose tail may need masking, if it is one of this CTA's
       const int last_rel = (n_kv_total - 1 - kv0) % kv_step == 0 ? (n_kv_total - 1 - kv0) / kv_step : -1;
       for (int j = 0; j < n_kv; ++j) {
-#ifdef CHITU_ATTN_TIMING
-        c0 = clock64();
-#endif
         mbar_wait(bar_s_full + 8 * t, j & 1, abort_flag, p.status, kDevTimeoutSoftmax);
         tc_fence_after_sync();
-        TICK(tw)
-        // Row of 128 scores into registers, 32 columns per load; the load of chunk
-        // c+1 is in flight while the running maximum of chunk c is taken.
-        uint32_t s[4][32];
-        const bool last_tile = (jt == last_rel && tail_valid < kTileN);
+        softmax_step<kFp16>(t_s, t_o, bar_p_full + 16 * t, j == 0, jt == last_rel ? tail_valid : kTileN, sl2, m_used, l_sum);
         if (++jt == n_kv) jt = 0;
-        float mx0 = -INFINITY, mx1 = -INFINITY;
-        tmem_ld32(t_s, s[0]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          tmem_wait_ld();
-          if (c < 3) tmem_ld32(t_s + (c + 1) * 32, s[c + 1]);
-          if (last_tile) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c * 32 + i >= tail_valid) s[c][i] = 0xff800000u;  // -inf
-          }
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            mx0 = max3(mx0, __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
-            mx1 = max3(mx1, __uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3]));
-          }
-        }
-        TICK(tl)
-        const float mx = fmaxf(mx0, mx1);
-
-        if (j == 0) {
-          m_used = mx;
-        } else {
-          const bool need = (mx - m_used) * sl2 > kRescaleThreshold;
-          if (__any_sync(0xffffffffu, need)) {
-            const float f = need ? fast_exp2((m_used - mx) * sl2) : 1.0f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t o[32];
-              tmem_ld32(t_o + c * 32, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-              tmem_st32(t_o + c * 32, o);
-            }
-            l_sum *= f;
-            if (need) m_used = mx;
-          }
-        }
-
-        // p = 2^(s*scale - m*scale): packed two-wide FMA / add, one MUFU per element
-        const float2 sl2_2 = make_float2(sl2, sl2);
-        const float neg_m = -m_used * sl2;
-        const float2 neg_m2 = make_float2(neg_m, neg_m);
-        uint32_t pk[2][32];
-        float2 la = make_float2(0.f, 0.f), lb = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            float2 x0 = __ffma2_rn(make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sl2_2, neg_m2);
-            float2 x1 =
-                __ffma2_rn(make_float2(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3])), sl2_2, neg_m2);
-            // kPolyPairs of every 8 pairs take the FMA-pipe polynomial, the rest the MUFU unit, so
-            // that both pipes stay busy (this iteration handles pairs 2g and 2g+1, g = i / 4)
-            constexpr int kPolyOdd = kPolyPairs < 4 ? kPolyPairs : 4;
-            constexpr int kPolyEven = kPolyPairs > 4 ? kPolyPairs - 4 : 0;
-            if (((i >> 2) & 3) < kPolyEven) {
-              x0 = exp2_poly2(x0);
-            } else {
-              x0.x = fast_exp2(x0.x);
-              x0.y = fast_exp2(x0.y);
-            }
-            if (((i >> 2) & 3) < kPolyOdd) {
-              x1 = exp2_poly2(x1);
-            } else {
-              x1.x = fast_exp2(x1.x);
-              x1.y = fast_exp2(x1.y);
-            }
-            la = __fadd2_rn(la, x0);
-            lb = __fadd2_rn(lb, x1);
-            pk[c >> 1][(c & 1) * 16 + (i >> 1)] = pack2<kFp16>(x0.x, x0.y);
-            pk[c >> 1][(c & 1) * 16 + (i >> 1) + 1] = pack2<kFp16>(x1.x, x1.y);
-            if ((c & 1) == 1 && i == 28) {
-              // 64 probabilities done: hand this half to the MMA warp
-              TICK(tm)
-              tmem_st32(t_s + (c >> 1) * 32, pk[c >> 1]);
-              tmem_wait_st();
-              tc_fence_before_sync();
-              mbar_arrive(bar_p_full + 16 * t + 8 * (c >> 1));
-              TICK(ts)
-            }
-          }
-        l_sum += (la.x + la.y) + (lb.x + lb.y);
       }
-#ifdef CHITU_ATTN_TIMING
-      if (p.dbg != nullptr && bx == 0 && by == 0 && bz == 0 && lane == 0 && (warp & 3) == 0) {
-        p.dbg[t * 4 + 0] = tw; p.dbg[t * 4 + 1] = tl; p.dbg[t * 4 + 2] = tm; p.dbg[t * 4 + 3] = ts;
-      }
-#endif
 
       // epilogue: O / l -> 16-bit, row-contiguous 256-byte stores; LSE in natural log
       if (t == 0 && row_in_tile == 0) CHITU_TRACE(3);
@@ -844,7 +838,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int batch = ez / p.n_splits;
       const int split = ez - batch * p.n_splits;
       const int row = qblock * (kQTiles * kTileM) + t * kTileM + row_in_tile;
-      const float inv_l = 1.0f / l_sum;
+      // no finite score at all: undefined over a whole row, no weight in a merge of key ranges
+      const bool empty = m_used == -INFINITY;
+      if (empty && p.n_splits == 1) l_sum = __int_as_float(0x7fffffff);
+      const float inv_l = empty && p.n_splits > 1 ? 0.f : 1.0f / l_sum;
       uint4* dst;
       const bool in_prefix = p.n_dest != 0 && row < p.prefix_rows;
       if (p.n_dest == 0) {

@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "attn_fwd.cuh"
+#include "attn_persist.cuh"
 #include "elementwise.cuh"
 #include "dit_elementwise.cuh"
 #include "quant.cuh"
@@ -156,6 +157,7 @@ struct OutScatter {
 
 struct KeySplit {
   int n_splits = 1;
+  bool balance = false;  // n_splits 1: the workspace may be used to cut the last wave's query blocks
   void* workspace = nullptr;
   int64_t workspace_bytes = 0;
 };
@@ -209,6 +211,111 @@ int64_t splitkv_workspace_bytes(int B, int Sq, int H, int D, int n_splits) {
   return kSplitHeaderBytes + static_cast<int64_t>(n_splits) * rows * (static_cast<int64_t>(D) + 1) * 4;
 }
 
+// Which kernel a plain call (local tensors, keys not split by the caller) takes, and how its query blocks are cut
+// (see AttnPersistParams).
+//
+// The blocks that do not fill the last wave of SMs - one CTA each - are cut into one bundle of key-tile steps per
+// SM, none shorter than an eighth of the keys (the CTA that completes a query block merges all its fragments).
+// A cut costs about kCutSteps steps (two epilogues to scratch memory instead of one to the output, and the merge).
+// Grids that do not fill the machine once are the business of the key-split entry points.
+//
+// Persistent CTAs save the five steps that a CTA of attn_fwd_kernel spends on starting and ending, but they drift
+// apart, while CTAs that start together stay together and have their reads of the same key tiles coalesced on
+// the way to L2 (S = 32760, H = 12: 460 M sectors read against 744 M, at the power limit 4.83 against 4.93 ms).
+// So long rows take the persistent kernel only where a cut gains more than that.  Measured, attn_fwd_kernel ->
+// persistent, us: 512 keys 147 -> 106 (S = 32760, H = 12); 36 key tiles 210 -> 206 (Flux, 2.9 waves);
+// 61 tiles cut 323 -> 302 (2.5 waves), 64 tiles cut 340 -> 329 (2.6 waves), uncut 340 -> 339;
+// 256 tiles cut 4835 -> 4835 (10.4 waves), uncut 4835 -> 4925.
+struct CutPlan {
+  bool persistent = true;
+  int cut_items = 0, n_bundles = 0, bundle_steps = 1;
+};
+constexpr int kCutSteps = 5;
+constexpr int kPersistentTiles = 64;
+CutPlan plan_cut(long long items, int n_kv, int sms, bool may_cut) {
+  CutPlan c;
+  c.persistent = n_kv <= kPersistentTiles;
+  if (sms <= 0 || !may_cut) return c;
+  const long long waves = items / sms, rem = items % sms;
+  if (waves == 0 || rem == 0) return c;
+  const long long per_sm = (rem * n_kv + sms - 1) / sms, floor_steps = (n_kv + 7) / 8;
+  const long long steps = per_sm > floor_steps ? per_sm : floor_steps;
+  const long long whole = (waves + 1) * n_kv, cut = waves * n_kv + steps + kCutSteps;
+  if (cut * 100 >= whole * (c.persistent ? 98 : 94)) return c;
+  c.persistent = true;
+  c.cut_items = static_cast<int>(rem);
+  c.bundle_steps = static_cast<int>(steps);
+  c.n_bundles = static_cast<int>((rem * n_kv + steps - 1) / steps);
+  return c;
+}
+int64_t cut_workspace_bytes(const CutPlan& c) {
+  if (c.cut_items == 0) return 0;
+  return kSplitHeaderBytes + static_cast<int64_t>(c.n_bundles) * 4 * chitu::kTileM * (chitu::kHeadDim + 1) * 4;
+}
+int current_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return sms;
+}
+long long query_blocks(int B, int Sq, int H) {
+  return static_cast<long long>((Sq + chitu::kQTiles * chitu::kTileM - 1) / (chitu::kQTiles * chitu::kTileM)) * B * H;
+}
+
+// A plain call on the persistent kernel.
+int attn_persist_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* out, float* lse,
+                        int B, int Sq, int Sk, int H, float scale_log2, bool fp16, const CutPlan& cut, void* workspace,
+                        int64_t workspace_bytes, int* status, cudaStream_t st) {
+  CUtensorMap to;
+  const int64_t out_strides[4] = {static_cast<int64_t>(Sq) * H * chitu::kHeadDim, static_cast<int64_t>(H) * chitu::kHeadDim,
+                                  chitu::kHeadDim, 1};
+  const int rc = make_qkv_map(&to, out, B, Sq, H, out_strides, "out", 32);
+  if (rc != CHITU_OK) return rc;
+  chitu::AttnPersistParams p;
+  p.lse = lse;
+  p.status = status;
+  p.B = B;
+  p.H = H;
+  p.Sq = Sq;
+  p.Sk = Sk;
+  p.scale_log2 = scale_log2;
+  p.n_kv = (Sk + chitu::kTileN - 1) / chitu::kTileN;
+  p.n_qblocks = (Sq + chitu::kQTiles * chitu::kTileM - 1) / (chitu::kQTiles * chitu::kTileM);
+  const long long items = query_blocks(B, Sq, H);
+  p.cut_items = cut.cut_items;
+  p.n_bundles = cut.n_bundles;
+  p.bundle_steps = cut.bundle_steps;
+  p.by_n_kv.set(p.n_kv);
+  p.by_n_qblocks.set(p.n_qblocks);
+  p.by_batch.set(B);
+  p.by_bundle_steps.set(cut.bundle_steps);
+  p.count = nullptr;
+  p.part_o = p.part_lse = nullptr;
+  if (cut.cut_items > 0) {
+    if ((reinterpret_cast<uintptr_t>(workspace) & 15) || workspace_bytes < cut_workspace_bytes(cut))
+      return fail(CHITU_E_INVALID, "attn_fwd: workspace must be 16-byte aligned and hold %lld bytes",
+                  (long long)cut_workspace_bytes(cut));
+    p.count = static_cast<int*>(workspace);
+    p.part_o = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kSplitHeaderBytes);
+    p.part_lse = p.part_o + static_cast<size_t>(cut.n_bundles) * 4 * chitu::kTileM * chitu::kHeadDim;
+  }
+  static bool attr_done[2][kMaxDevices] = {};
+  static std::mutex attr_mu;
+  const cudaError_t attr_err =
+      fp16 ? ensure_dynamic_smem(chitu::attn_persist_kernel<true>, chitu::kPersistSmemBytes, attr_done[1], attr_mu)
+           : ensure_dynamic_smem(chitu::attn_persist_kernel<false>, chitu::kPersistSmemBytes, attr_done[0], attr_mu);
+  if (attr_err != cudaSuccess) return cuda_fail(attr_err, "attn_fwd: cudaFuncSetAttribute");
+  const dim3 grid(static_cast<unsigned>(items - cut.cut_items + cut.n_bundles));
+  if (fp16)
+    chitu::attn_persist_kernel<true><<<grid, chitu::kAttnThreads, chitu::kPersistSmemBytes, st>>>(tq, tk, tv, to, p);
+  else
+    chitu::attn_persist_kernel<false><<<grid, chitu::kAttnThreads, chitu::kPersistSmemBytes, st>>>(tq, tk, tv, to, p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "attn_fwd: launch");
+  return CHITU_OK;
+}
+
 int attn_fwd_impl(const void* q, const void* k, const void* v, void* out, const OutScatter& sc, float* lse, int B,
                   int Sq, int Sk, int H, int D, const int64_t* q_strides, const int64_t* k_strides,
                   const int64_t* v_strides, float softmax_scale, int dtype, int* status, void* stream,
@@ -257,6 +364,16 @@ int attn_fwd_impl(const void* q, const void* k, const void* v, void* out, const 
   if ((rc = make_qkv_map(&tq, q, B, Sq, H, q_strides, "q")) != CHITU_OK) return rc;
   if ((rc = make_qkv_map(&tk, k, B, Sk, H, k_strides, "k")) != CHITU_OK) return rc;
   if ((rc = make_qkv_map(&tv, v, B, Sk, H, v_strides, "v")) != CHITU_OK) return rc;
+
+  if (n_splits == 1 && sc.n_dest == 0 && ex.sync == nullptr && qpre == nullptr) {
+    const long long items = query_blocks(B, Sq, H);
+    const int n_kv = (Sk + chitu::kTileN - 1) / chitu::kTileN;
+    const CutPlan cut = plan_cut(items, n_kv, current_sms(), ks.balance && ks.workspace != nullptr);
+    if (cut.persistent && items * n_kv < (1LL << 31))  // (the kernel numbers key-tile steps with 31 bits)
+      return attn_persist_launch(tq, tk, tv, out, lse, B, Sq, Sk, H, softmax_scale * 1.4426950408889634f,
+                                 dtype == CHITU_DTYPE_FP16, cut, ks.workspace, ks.workspace_bytes, status,
+                                 static_cast<cudaStream_t>(stream));
+  }
 
   chitu::AttnParams p;
   p.out = out;
@@ -498,6 +615,23 @@ int chitu_b200_attn_fwd(const void* q, const void* k, const void* v, void* out, 
                         float softmax_scale, int dtype, int* status, void* stream) {
   return attn_fwd_impl(q, k, v, out, OutScatter{}, lse, B, Sq, Sk, H, D, q_strides, k_strides, v_strides,
                        softmax_scale, dtype, status, stream);
+}
+
+int64_t chitu_b200_attn_balanced_workspace_bytes(int B, int Sq, int Sk, int H) {
+  if (B <= 0 || Sq <= 0 || Sk <= 0 || H <= 0) return 0;
+  return cut_workspace_bytes(plan_cut(query_blocks(B, Sq, H), (Sk + chitu::kTileN - 1) / chitu::kTileN, current_sms(), true));
+}
+
+int chitu_b200_attn_fwd_balanced(const void* q, const void* k, const void* v, void* out, float* lse, int B, int Sq,
+                                 int Sk, int H, int D, const int64_t* q_strides, const int64_t* k_strides,
+                                 const int64_t* v_strides, float softmax_scale, int dtype, void* workspace,
+                                 int64_t workspace_bytes, int* status, void* stream) {
+  KeySplit ks;
+  ks.balance = true;
+  ks.workspace = workspace;
+  ks.workspace_bytes = workspace_bytes;
+  return attn_fwd_impl(q, k, v, out, OutScatter{}, lse, B, Sq, Sk, H, D, q_strides, k_strides, v_strides,
+                       softmax_scale, dtype, status, stream, ks);
 }
 
 int64_t chitu_b200_attn_splitkv_workspace_bytes(int B, int Sq, int H, int D, int n_splits) {

@@ -216,7 +216,8 @@ def attn_fwd(
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device) if return_lse else None
     scale = float(softmax_scale) if softmax_scale is not None else 1.0 / math.sqrt(D)
     lib = _lib.load()
-    if n_splits is None:
+    automatic = n_splits is None
+    if automatic:
         n_splits = auto_key_splits(B, Sq, Sk, H)
     if q_pre is not None:
         import ctypes
@@ -260,10 +261,19 @@ def attn_fwd(
                 ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), _stream_ptr(q.device),
             )
         else:
-            rc = lib.chitu_b200_attn_fwd(
+            # the query blocks of a partly filled last wave are cut along the keys; a graph being captured
+            # keeps them whole (the scratch belongs to eager calls of this stream, which may run beside a replay)
+            ws_ptr, ws_bytes = None, 0
+            if automatic and not torch.cuda.is_current_stream_capturing():
+                need = int(lib.chitu_b200_attn_balanced_workspace_bytes(B, Sq, Sk, H))
+                if need:
+                    ws = splitkv_workspace(q.device, need) if workspace is None else workspace
+                    if ws.numel() * ws.element_size() >= need and ws.device == q.device:
+                        ws_ptr, ws_bytes = ws.data_ptr(), ws.numel() * ws.element_size()
+            rc = lib.chitu_b200_attn_fwd_balanced(
                 q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                 lse.data_ptr() if lse is not None else None, B, Sq, Sk, H, D, _lib.i64_array(q.stride()),
-                _lib.i64_array(k.stride()), _lib.i64_array(v.stride()), scale, _DTYPES[q.dtype],
+                _lib.i64_array(k.stride()), _lib.i64_array(v.stride()), scale, _DTYPES[q.dtype], ws_ptr, ws_bytes,
                 status_word(q.device).data_ptr(), _stream_ptr(q.device),
             )
     _lib.check(rc, "attn_fwd")

@@ -1,0 +1,99 @@
+"""The persistent attention kernel: several query blocks per CTA, and blocks cut along the keys and merged.
+
+Tolerances as in test_gpu_attention.py (bf16 inputs, fp32 oracle on the same inputs); two schedules of the same
+arithmetic differ by the 16-bit rounding of the result (2^-8 relative) at most.
+"""
+
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B, Sq, Sk, H, dtype, seed):
+    gen = torch.Generator().manual_seed(seed)
+    return (torch.randn(B, Sq, H, 128, generator=gen).to(dtype), torch.randn(B, Sk, H, 128, generator=gen).to(dtype),
+            torch.randn(B, Sk, H, 128, generator=gen).to(dtype))
+
+
+def _need(B, Sq, Sk, H):
+    from chitudiffusion_b200 import _lib
+
+    return int(_lib.load().chitu_b200_attn_balanced_workspace_bytes(B, Sq, Sk, H))
+
+
+# (B, Sq, Sk, H, dtype, cut): one key tile per block (masked and full); many blocks per CTA; a last block of one tile;
+# cut last waves whose bundles start inside, end inside and span two blocks
+@pytest.mark.parametrize("B,Sq,Sk,H,dtype,cut", [
+    (1, 2500, 77, 40, torch.bfloat16, False),
+    (2, 1100, 128, 37, torch.float16, False),
+    (1, 4097, 129, 24, torch.bfloat16, False),
+    (1, 1100, 1500, 37, torch.bfloat16, True),
+    (1, 1300, 1409, 26, torch.float16, True),
+    (2, 513, 2049, 50, torch.bfloat16, True),
+])
+def test_matches_the_oracle(B, Sq, Sk, H, dtype, cut):
+    from chitudiffusion_b200 import ops
+
+    q, k, v = _inputs(B, Sq, Sk, H, dtype, Sq + Sk)
+    ref, ref_lse = oracle.sdpa_fp32(q, k, v, return_lse=True)
+    assert (_need(B, Sq, Sk, H) > 0) == cut
+    qc, kc, vc = q.cuda(), k.cuda(), v.cuda()
+    ws = torch.zeros(max(_need(B, Sq, Sk, H), 65536), dtype=torch.uint8, device="cuda")
+    for _ in range(2):  # the second call finds the first one's scratch
+        out, lse = ops.attn_fwd(qc, kc, vc, return_lse=True, workspace=ws)
+        assert (out.float().cpu() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item()
+        assert (lse.cpu() - ref_lse).abs().max().item() <= 1e-3
+    assert int(ws[:65536].max().item()) == 0  # the counters are back at zero
+    whole, lse1 = ops.attn_fwd(qc, kc, vc, return_lse=True, n_splits=1)
+    assert (out.float() - whole.float()).abs().max().item() <= 2 ** -7 * ref.abs().max().item()
+    assert (lse - lse1).abs().max().item() <= 1e-4
+    ops.check_status()
+
+
+def test_a_fragment_without_a_finite_score_carries_no_weight():
+    """Keys whose scores are -inf for every row: wherever the cuts fall, the others decide alone."""
+    from chitudiffusion_b200 import ops
+
+    q, k, v = _inputs(1, 1100, 1500, 37, torch.bfloat16, 3)
+    q[..., 0] = 1.0
+    for lo, hi in ((0, 700), (900, 1500), (128, 256)):
+        kk = k.clone()
+        kk[:, lo:hi, :, 0] = float("-inf")
+        keep = torch.tensor([i for i in range(1500) if not lo <= i < hi])
+        ref, ref_lse = oracle.sdpa_fp32(q, kk[:, keep], v[:, keep], return_lse=True)
+        for n_splits in (None, 1, 2, 3):
+            out, lse = ops.attn_fwd(q.cuda(), kk.cuda(), v.cuda(), return_lse=True, n_splits=n_splits)
+            assert (out.float().cpu() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item()
+            assert (lse.cpu() - ref_lse).abs().max().item() <= 1e-3
+
+
+def test_a_row_without_any_finite_score_is_undefined():
+    from chitudiffusion_b200 import ops
+
+    q, k, v = _inputs(1, 1100, 1500, 37, torch.bfloat16, 5)
+    q[..., 0] = 1.0
+    k[..., 0] = float("-inf")
+    for n_splits in (None, 1, 3):
+        out, _ = ops.attn_fwd(q.cuda(), k.cuda(), v.cuda(), n_splits=n_splits)
+        assert torch.isnan(out).all()
+
+
+def test_a_captured_call_keeps_its_query_blocks_whole():
+    """Inside a capture no scratch of the stream is used: a replay may run beside eager calls that use it."""
+    from chitudiffusion_b200 import ops
+
+    q, k, v = (t.cuda() for t in _inputs(1, 1100, 1500, 37, torch.bfloat16, 4))
+    whole, _ = ops.attn_fwd(q, k, v, n_splits=1)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ops.attn_fwd(q, k, v)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out, _ = ops.attn_fwd(q, k, v)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, whole)
