@@ -273,7 +273,12 @@ def ptr_array(ptrs: Sequence[int]):
     return (ctypes.c_void_p * len(ptrs))(*[int(p) for p in ptrs])
 
 
+_I64x4 = ctypes.c_int64 * 4
+
+
 def i64_array(values: Sequence[int]):
+    if len(values) == 4:
+        return _I64x4(*values)
     return (ctypes.c_int64 * len(values))(*[int(v) for v in values])
 
 

@@ -547,7 +547,7 @@ __global__ void peer_barrier_kernel(const PeerBarrierParams p) {
       asm volatile("ld.acquire.sys.global.s32 %0, [%1];" : "=r"(seen) : "l"(mine) : "memory");
       if (seen - epoch >= 0) break;  // epochs only grow (wrap-safe comparison)
       if ((++spins & 0xff) == 0 && clock64() - t0 > p.timeout_cycles) {
-        if (p.status) atomicCAS(p.status, 0, 5);
+        record_status(p.status, 5);
         break;
       }
     }

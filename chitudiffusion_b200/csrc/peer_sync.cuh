@@ -35,6 +35,15 @@
 
 namespace chitu {
 
+// First come, first recorded.  The status word may be host memory that the device addresses, where an atomic would
+// depend on what the link to the host supports; two waits that run out at once leave either code, and that is enough.
+__device__ __forceinline__ void record_status(int* status, int code) {
+  if (status == nullptr) return;
+  volatile int* word = status;
+  if (*word == 0) *word = code;
+  __threadfence_system();
+}
+
 constexpr int kSyncInts = 64;
 constexpr int kSyncInFlag = 16, kSyncInEpoch = 24, kSyncScatterDone = 25;
 constexpr int kSyncOutFlag = 32, kSyncOutEpoch = 40, kSyncAttnDone = 41, kSyncWaitEpoch = 42;
@@ -96,7 +105,7 @@ __device__ __forceinline__ bool wait_flag(const int* flag, int epoch, long long 
     unsigned spins = 0;
     while (ld_acquire_sys(flag) - epoch < 0) {
       if ((++spins & 0x3f) == 0 && clock64() - t0 > timeout_cycles) {
-        if (status) atomicCAS(status, 0, 5);
+        record_status(status, 5);
         return false;
       }
     }

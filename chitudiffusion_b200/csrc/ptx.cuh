@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "peer_sync.cuh"
+
 namespace chitu {
 
 // Status words written to the caller-provided device int (0 = ok).
@@ -78,7 +80,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
       if (*abort_flag) return false;
       if (clock64() - t0 > CHITU_WAIT_CYCLES) {
         *abort_flag = 1;
-        if (status) atomicCAS(status, 0, code);
+        record_status(status, code);
         return false;
       }
     }

@@ -7,6 +7,8 @@ on a CUDA device - there is no CPU path.
 
 from __future__ import annotations
 
+import ctypes
+import functools
 import math
 import os
 from typing import Optional, Sequence, Tuple
@@ -37,7 +39,27 @@ def _launched(n: int = 1) -> None:
 
 
 def _stream_ptr(device: torch.device) -> int:
-    return int(torch.cuda.current_stream(device).cuda_stream)
+    # the handle alone: building a torch Stream object costs ten times as much and every call needs it
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_GUARD = _NoGuard()
+
+
+def _on(device: torch.device):
+    """``torch.cuda.device(device)`` where that changes anything (entering and leaving it costs some microseconds)."""
+    if device.index is None or torch._C._cuda_getDevice() == device.index:
+        return _NO_GUARD
+    return torch.cuda.device(device)
 
 
 def _require_cuda(*tensors: torch.Tensor) -> None:
@@ -46,63 +68,56 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
             raise RuntimeError("chitudiffusion_b200 runs on CUDA tensors only (there is no CPU path)")
 
 
+def _device_key(device) -> int:
+    index = torch.device(device).index if not isinstance(device, torch.device) else device.index
+    return torch.cuda.current_device() if index is None else index
+
+
 def status_word(device: torch.device) -> torch.Tensor:
-    """Per-device int32 status word that kernels with bounded waits report into."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    word = _status_words.get(key)
-    if word is None:
-        word = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
-        _status_words[key] = word
-    return word
+    """Per-device int32 status word that kernels with bounded waits report into.
+
+    It lives in pinned host memory, which kernels address directly: a wait that ran out is stored there and the host
+    looks at it without a copy, an event or a synchronisation in between.
+    """
+    key = _device_key(device)
+    entry = _status_words.get(key)
+    if entry is None:
+        word = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        entry = _status_words.setdefault(key, (word, ctypes.c_int32.from_address(word.data_ptr())))
+    return entry[0]
+
+
+def _take_status(key: int) -> None:
+    """Raise (and clear the word) if it is set."""
+    entry = _status_words.get(key)
+    if entry is not None and entry[1].value != 0:
+        code = entry[1].value
+        entry[1].value = 0
+        raise _lib.ChituB200Error(f"device status {code}: {_STATUS_NAMES.get(code, 'unknown')}")
 
 
 def check_status(device: Optional[torch.device] = None) -> None:
     """Synchronise and raise if any kernel on `device` reported a timed-out wait."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    word = status_word(dev)
-    code = int(word.item())
-    if code != 0:
-        word.zero_()
-        raise _lib.ChituB200Error(f"device status {code}: {_STATUS_NAMES.get(code, 'unknown')}")
-
-
-_status_mirrors = {}
+    key = torch.cuda.current_device() if device is None else _device_key(device)
+    torch.cuda.synchronize(key)
+    _take_status(key)
 
 
 def poll_status(device: Optional[torch.device] = None) -> None:
     """Deferred, non-blocking form of :func:`check_status` for the product path.
 
-    Each call first looks at the copy of the status word that the PREVIOUS call sent to pinned host
-    memory (if that copy has landed) and raises when it is non-zero, then enqueues a fresh copy behind
-    the work just launched.  A timed-out device wait therefore surfaces as an exception one call later
-    instead of as silently wrong output, and no call ever synchronises.  ``CHITU_B200_CHECK=1`` makes
-    every poll a full synchronising check.  Nothing is enqueued while the stream is being captured.
+    Looks at the status word as it is: a device wait that timed out surfaces as an exception at the first call after
+    its kernel has reported it, instead of as silently wrong output, and no call ever synchronises or enqueues
+    anything.  ``CHITU_B200_CHECK=1`` makes every poll a full synchronising check.  Does nothing while the stream is
+    being captured.
     """
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    if torch.cuda.is_current_stream_capturing():
-        return  # event queries and host copies have no place inside a capture
-    if os.environ.get("CHITU_B200_CHECK", "0") == "1":
-        check_status(dev)
-        return
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
-    mirror = _status_mirrors.get(key)
-    if mirror is None:
-        mirror = {"host": torch.zeros(1, dtype=torch.int32).pin_memory(), "event": None}
-        _status_mirrors[key] = mirror
-    ev = mirror["event"]
-    if ev is not None and ev.query():
-        code = int(mirror["host"][0])
-        if code != 0:
-            mirror["host"].zero_()
-            mirror["event"] = None
-            status_word(dev).zero_()
-            raise _lib.ChituB200Error(f"device status {code}: {_STATUS_NAMES.get(code, 'unknown')}")
-    if ev is None or ev.query():
-        mirror["host"].copy_(status_word(dev), non_blocking=True)
-        if ev is None:
-            ev = torch.cuda.Event()
-            mirror["event"] = ev
-        ev.record(torch.cuda.current_stream(dev))
+    key = torch.cuda.current_device() if device is None else _device_key(device)
+    entry = _status_words.get(key)
+    checking = os.environ.get("CHITU_B200_CHECK", "0") == "1"
+    if (checking or (entry is not None and entry[1].value != 0)) and not torch.cuda.is_current_stream_capturing():
+        if checking:
+            torch.cuda.synchronize(key)
+        _take_status(key)
 
 
 def set_flag_wait_cycles(cycles: int) -> int:
@@ -122,14 +137,15 @@ def auto_key_splits(B: int, Sq: int, Sk: int, H: int) -> int:
     143 us) plus about one tile step per range for the merge.  The split that minimises it is taken when it
     saves at least 8 %: it fills small grids (54 CTAs -> 2 ranges).
     ``CHITU_B200_KEY_SPLITS`` overrides."""
-    import os
-
     forced = os.environ.get("CHITU_B200_KEY_SPLITS")
     tiles = -(-Sk // 128)
     if forced:
         return max(1, min(int(forced), tiles, 64))
-    ctas = -(-Sq // 256) * H * B
+    return _wave_model_splits(-(-Sq // 256) * H * B, tiles)
 
+
+@functools.lru_cache(maxsize=1024)
+def _wave_model_splits(ctas: int, tiles: int) -> int:
     def cost(n):
         per = -(-tiles // n)
         n_eff = -(-tiles // per)
@@ -171,6 +187,12 @@ def splitkv_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 def splitkv_workspace_bytes(B: int, Sq: int, H: int, D: int, n_splits: int) -> int:
     """Bytes of scratch a key-split call of this shape needs (0 for one split)."""
     return int(_lib.load().chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, int(n_splits)))
+
+
+@functools.lru_cache(maxsize=1024)
+def _balanced_workspace_bytes(device_index: int, B: int, Sq: int, Sk: int, H: int) -> int:
+    with torch.cuda.device(device_index):
+        return int(_lib.load().chitu_b200_attn_balanced_workspace_bytes(B, Sq, Sk, H))
 
 
 def attn_fwd(
@@ -220,8 +242,6 @@ def attn_fwd(
     if automatic:
         n_splits = auto_key_splits(B, Sq, Sk, H)
     if q_pre is not None:
-        import ctypes
-
         w, rstd, table = q_pre.get("weight"), q_pre.get("rstd"), q_pre.get("rope_table")
         _require_cuda(w, rstd, table)
         if w is not None:
@@ -239,7 +259,7 @@ def attn_fwd(
             need = int(lib.chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, n_splits))
             ws = workspace if workspace is not None else splitkv_workspace(q.device, need)
             ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()
-        with torch.cuda.device(q.device):
+        with _on(q.device):
             rc = lib.chitu_b200_attn_fwd_qpre(
                 q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr() if lse is not None else None,
                 B, Sq, Sk, H, D, _lib.i64_array(q.stride()), _lib.i64_array(k.stride()), _lib.i64_array(v.stride()),
@@ -248,7 +268,7 @@ def attn_fwd(
         _lib.check(rc, "attn_fwd_qpre")
         _launched(1)
         return out, lse
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         if n_splits > 1:
             need = int(lib.chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, n_splits))
             ws = workspace if workspace is not None else splitkv_workspace(q.device, need)
@@ -265,7 +285,7 @@ def attn_fwd(
             # keeps them whole (the scratch belongs to eager calls of this stream, which may run beside a replay)
             ws_ptr, ws_bytes = None, 0
             if automatic and not torch.cuda.is_current_stream_capturing():
-                need = int(lib.chitu_b200_attn_balanced_workspace_bytes(B, Sq, Sk, H))
+                need = _balanced_workspace_bytes(q.device.index, B, Sq, Sk, H)
                 if need:
                     ws = splitkv_workspace(q.device, need) if workspace is None else workspace
                     if ws.numel() * ws.element_size() >= need and ws.device == q.device:
@@ -308,7 +328,7 @@ def attn_fwd_q8(
     need = int(lib.chitu_b200_attn_q8_workspace_bytes(B, Sq, Sk, H))
     ws = torch.empty(need + 256, dtype=torch.uint8, device=q.device)
     base = (ws.data_ptr() + 255) // 256 * 256
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = lib.chitu_b200_attn_fwd_q8(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr() if lse is not None else None,
             B, Sq, Sk, H, D, _lib.i64_array(q.stride()), _lib.i64_array(k.stride()), _lib.i64_array(v.stride()),
@@ -345,7 +365,7 @@ def lse_combine(
     if final_out is not None and (final_out.shape != block_out.shape or not final_out.is_contiguous()):
         raise ValueError("final_out must be contiguous [B,S,H,D]")
     lib = _lib.load()
-    with torch.cuda.device(acc_out.device):
+    with _on(acc_out.device):
         rc = lib.chitu_b200_lse_combine(
             acc_out.data_ptr(), acc_lse.data_ptr(), block_out.data_ptr(), block_lse.data_ptr(), B, S, H, D,
             _DTYPES[block_out.dtype], 1 if first else 0,
@@ -407,8 +427,6 @@ def qk_norm_rope(
     elif out_strides is None or heads_per_group is None:
         raise ValueError("out needs out_strides and heads_per_group")
     lib = _lib.load()
-    import ctypes
-
     split = (ctypes.c_int * 2)(int(axis_split[0]), int(axis_split[1]))
     common = (
         x.data_ptr(), _DTYPES[x.dtype], x.stride(1), weight.data_ptr() if weight is not None else None,
@@ -419,7 +437,7 @@ def qk_norm_rope(
     )
     tail = (_lib.i64_array(out_strides), int(heads_per_group), B, S, num_heads, D, 1 if round_mid else 0,
             _stream_ptr(x.device))
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         if out_ptrs is not None:
             rc = lib.chitu_b200_qk_norm_rope_scatter(*common, _lib.ptr_array(out_ptrs), len(out_ptrs),
                                                      _DTYPES[out_dtype], *tail)
@@ -457,8 +475,6 @@ def qk_norm_rope_batch(
     ``[B,S,H,D]`` result is allocated).  All jobs share dtype, shape and placement.  Returns the list
     of output tensors (``None`` for jobs written through ``out_ptrs``).
     """
-    import ctypes
-
     x0 = jobs[0]["x"]
     B, S, C = x0.shape
     D = C // num_heads
@@ -517,12 +533,10 @@ def qk_norm_rope_batch(
         split, int(pos_offset), _DTYPES[out_dtype], _lib.i64_array(out_strides), int(heads_per_group),
         B, S, num_heads, D, 1 if round_mid else 0,
     )
-    with torch.cuda.device(x0.device):
+    with _on(x0.device):
         if sync is not None:
-            import ctypes as _ct
-
             fn = lib.chitu_b200_qk_norm_rope_batch_stage if stage_only else lib.chitu_b200_qk_norm_rope_batch_signal
-            rc = fn(*args, _ct.byref(sync[0]), _stream_ptr(x0.device))
+            rc = fn(*args, ctypes.byref(sync[0]), _stream_ptr(x0.device))
         else:
             rc = lib.chitu_b200_qk_norm_rope_batch(*args, _stream_ptr(x0.device))
     _lib.check(rc, "qk_norm_rope_batch")
@@ -537,7 +551,7 @@ def strided_copy(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
         raise ValueError("strided_copy: src must be 5-d with a contiguous last dim, dst contiguous of the same shape")
     es = src.element_size()
     lib = _lib.load()
-    with torch.cuda.device(src.device):
+    with _on(src.device):
         rc = lib.chitu_b200_strided_copy(
             src.data_ptr(), dst.data_ptr(), *[int(n) for n in src.shape[:4]], int(src.shape[4]) * es,
             _lib.i64_array([s * es for s in src.stride()[:4]]), _stream_ptr(src.device),
@@ -567,7 +581,7 @@ def layernorm_modulate(x: torch.Tensor, mul: Optional[torch.Tensor] = None, add:
     (m, ms), (a, as_) = vec(mul), vec(add)
     out = torch.empty((B, L, C), dtype=out_dtype, device=x.device)
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib.chitu_b200_layernorm_modulate(
             x.data_ptr(), _DTYPES[x.dtype], out.data_ptr(), _DTYPES[out_dtype], B * L, L, C,
             m.data_ptr() if m is not None else None, ms,
@@ -590,7 +604,7 @@ def gate_residual(x: torch.Tensor, y: torch.Tensor, gate: Optional[torch.Tensor]
             raise ValueError("gate_residual: gate must be fp32 with C channels for 1 or B batches")
         gs = g.stride(0) if g.shape[0] == B and B > 1 else 0
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         rc = lib.chitu_b200_gate_residual(x.data_ptr(), _DTYPES[x.dtype], y.data_ptr(), _DTYPES[y.dtype], B * L, L, C,
                                           g.data_ptr() if g is not None else None, gs, _stream_ptr(x.device))
     _lib.check(rc, "gate_residual")
@@ -607,7 +621,7 @@ def cfg_combine(cond: torch.Tensor, uncond: torch.Tensor, scale: float, rescale:
     out = torch.empty_like(cond)
     C = cond.shape[-1]
     lib = _lib.load()
-    with torch.cuda.device(cond.device):
+    with _on(cond.device):
         rc = lib.chitu_b200_cfg_combine(cond.data_ptr(), uncond.data_ptr(), out.data_ptr(), _DTYPES[cond.dtype],
                                         cond.numel() // C, C, float(scale), int(rescale), _stream_ptr(cond.device))
     _lib.check(rc, "cfg_combine")
@@ -619,7 +633,7 @@ def peer_copy_2d(dst_ptr: int, dst_pitch: int, src_ptr: int, src_pitch: int, wid
                  device: torch.device) -> None:
     """``rows`` pieces of ``width`` bytes between device buffers (either may be peer-mapped), on the copy engines."""
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         rc = lib.chitu_b200_peer_copy_2d(int(dst_ptr), int(dst_pitch), int(src_ptr), int(src_pitch), int(width),
                                          int(rows), _stream_ptr(device))
     _lib.check(rc, "peer_copy_2d")
@@ -633,7 +647,7 @@ def scatter_rows(src: torch.Tensor, dst_ptrs: Sequence[int], rows: int, dst_batc
         raise ValueError("scatter_rows: src must be contiguous [B, n_dest*rows, ...]")
     row_bytes = src[0, 0].numel() * src.element_size()
     lib = _lib.load()
-    with torch.cuda.device(src.device):
+    with _on(src.device):
         rc = lib.chitu_b200_scatter_rows(src.data_ptr(), _lib.ptr_array(dst_ptrs), len(dst_ptrs), int(src.shape[0]),
                                          int(rows), int(row_bytes), int(dst_batch_stride_bytes),
                                          int(dst_row_stride_bytes), _stream_ptr(src.device))
@@ -671,7 +685,7 @@ def attn_fwd_scatter(
         if ws.numel() * ws.element_size() < need or ws.device != q.device:
             raise ValueError(f"attn_fwd_scatter: workspace must hold {need} bytes on {q.device}")
         ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = lib.chitu_b200_attn_fwd_scatter(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr_array(out_ptrs), len(out_ptrs), int(rows_per_dest),
             int(dest_batch_stride), int(dest_row_stride), int(dest_head_offset), None, B, Sq, Sk, H, D,
@@ -686,7 +700,7 @@ def attn_fwd_scatter(
 def peer_barrier(flag_ptrs: Sequence[int], rank: int, world: int, device: torch.device) -> None:
     """Enqueue the bounded cross-GPU barrier on the current stream; see ``chitu_b200_peer_barrier``."""
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         rc = lib.chitu_b200_peer_barrier(_lib.ptr_array(flag_ptrs), int(rank), int(world),
                                          status_word(device).data_ptr(), _stream_ptr(device))
     _lib.check(rc, "peer_barrier")
@@ -717,8 +731,6 @@ def attn_fwd_exchange(
     """:func:`attn_fwd_scatter` over exchange buffers guarded by arrival flags; see ``chitu_b200_attn_fwd_exchange``.
     With ``push`` (a ``_lib.push_desc`` pair) the launch also delivers the staged rows to the peers
     (``chitu_b200_attn_fwd_exchange_push``)."""
-    import ctypes
-
     _require_cuda(q, k, v)
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
@@ -738,7 +750,7 @@ def attn_fwd_exchange(
     if push is not None:
         if prefix_rows:
             raise NotImplementedError("push mode has no replicated prefix")
-        with torch.cuda.device(q.device):
+        with _on(q.device):
             rc = lib.chitu_b200_attn_fwd_exchange_push(
                 q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr_array(out_ptrs), len(out_ptrs),
                 int(rows_per_dest), int(dest_batch_stride), int(dest_row_stride), int(dest_head_offset), B, Sq, Sk, H,
@@ -749,7 +761,7 @@ def attn_fwd_exchange(
         _lib.check(rc, "attn_fwd_exchange_push")
         _launched(1)
         return
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         rc = lib.chitu_b200_attn_fwd_exchange(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), _lib.ptr_array(out_ptrs), len(out_ptrs), int(rows_per_dest),
             int(dest_batch_stride), int(dest_row_stride), int(dest_head_offset), B, Sq, Sk, H, D,
@@ -776,7 +788,7 @@ def stamp(slots: torch.Tensor, index: int) -> None:
         raise ValueError("stamp: slots must be a contiguous int64 CUDA tensor")
     if not 0 <= index < slots.numel():
         raise IndexError("stamp: index out of range")
-    with torch.cuda.device(slots.device):
+    with _on(slots.device):
         rc = _lib.load().chitu_b200_stamp(slots.data_ptr() + 8 * int(index), _stream_ptr(slots.device))
     _lib.check(rc, "stamp")
 
@@ -788,10 +800,8 @@ def push_ctas(B: int, Sq: int, H: int, n_splits: int) -> int:
 
 def peer_wait_outputs(sync, device: torch.device) -> None:
     """Enqueue the bounded wait for every rank's output flag; see ``chitu_b200_peer_wait_outputs``."""
-    import ctypes
-
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         rc = lib.chitu_b200_peer_wait_outputs(ctypes.byref(sync[0]), status_word(device).data_ptr(), _stream_ptr(device))
     _lib.check(rc, "peer_wait_outputs")
     _launched()
