@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -773,9 +774,22 @@ int chitu_b200_lse_combine(float* acc_out, float* acc_lse, const void* block_out
        reinterpret_cast<uintptr_t>(final_out)) & 15)
     return fail(CHITU_E_INVALID, "lse_combine: buffers must be 16-byte aligned");
   const long long rows = static_cast<long long>(B) * S * H;
-  const int grid = grid_for(rows, 8, 148 * 16);
-  chitu::lse_combine_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      acc_out, acc_lse, block_out, block_lse, B, S, H, D, block_dtype, first, final_out, final_dtype);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (D == 128 && block_dtype != CHITU_DTYPE_FP32 && !final_out && rows < (1LL << 30)) {
+    const int grid = grid_for(rows, 8 * chitu::kCombineRows, 148 * 16);
+#define CHITU_COMBINE(FP16) \
+    (first ? chitu::lse_combine_d128_kernel<FP16, true><<<grid, 256, 0, st>>>(acc_out, acc_lse, block_out, block_lse, S, H, static_cast<int>(rows)) \
+           : chitu::lse_combine_d128_kernel<FP16, false><<<grid, 256, 0, st>>>(acc_out, acc_lse, block_out, block_lse, S, H, static_cast<int>(rows)))
+    if (block_dtype == CHITU_DTYPE_FP16)
+      CHITU_COMBINE(true);
+    else
+      CHITU_COMBINE(false);
+#undef CHITU_COMBINE
+  } else {
+    const int grid = grid_for(rows, 8, 148 * 16);
+    chitu::lse_combine_kernel<<<grid, 256, 0, st>>>(acc_out, acc_lse, block_out, block_lse, B, S, H, D, block_dtype, first,
+                                                    final_out, final_dtype);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "lse_combine: launch");
   return CHITU_OK;
@@ -1114,16 +1128,29 @@ int chitu_b200_layernorm_modulate(const void* x, int x_dtype, void* out, int out
   p.eps = eps;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int per_vec = x_dtype == CHITU_DTYPE_FP32 ? 4 : 8;
-  if (C % (32 * per_vec) == 0 && C / per_vec / 32 <= chitu::kLnWarpMaxVec &&
+  const int64_t batches = rows / rows_per_batch;
+  // the column form wants whole 16-byte vectors, whole batches and a block's worth of columns (narrow rows would leave
+  // most of its threads idle)
+  const int n_vec = C / per_vec;
+  if (C % per_vec == 0 && n_vec >= 64 && n_vec <= 2048 && rows % rows_per_batch == 0 && batches <= 65535 &&
       !(reinterpret_cast<uintptr_t>(out) & 15)) {
-    // rows of at most 8 KiB: one warp per row, eight rows per CTA
-    const int grid = static_cast<int>(std::min<int64_t>((rows + 7) / 8, 148 * 8));
+    const int two = n_vec > 1024;
+    const int threads = ((two ? (n_vec + 1) / 2 : n_vec) + 31) / 32 * 32;
+    const int rows_each = threads <= 384 ? 4 : 2;
+    const int64_t groups = (rows_per_batch + rows_each - 1) / rows_each;
+    const int64_t resident = std::max<int64_t>(1, 148 * (threads <= 384 ? (x_dtype == CHITU_DTYPE_FP32 ? 1152 : 768) / threads : 1) / batches);
+    const dim3 grid(static_cast<unsigned>(std::min<int64_t>(groups, resident)), static_cast<unsigned>(batches));
+#define CHITU_LN(DT) \
+    (two              ? chitu::layernorm_affine_rows_kernel<DT, 2, 1024><<<grid, threads, 0, st>>>(p) \
+     : threads <= 384 ? chitu::layernorm_affine_rows_kernel<DT, 1, 384><<<grid, threads, 0, st>>>(p) \
+                      : chitu::layernorm_affine_rows_kernel<DT, 1, 1024><<<grid, threads, 0, st>>>(p))
     if (x_dtype == CHITU_DTYPE_BF16)
-      chitu::layernorm_affine_warp_kernel<0><<<grid, 256, 0, st>>>(p);
+      CHITU_LN(0);
     else if (x_dtype == CHITU_DTYPE_FP16)
-      chitu::layernorm_affine_warp_kernel<1><<<grid, 256, 0, st>>>(p);
+      CHITU_LN(1);
     else
-      chitu::layernorm_affine_warp_kernel<2><<<grid, 256, 0, st>>>(p);
+      CHITU_LN(2);
+#undef CHITU_LN
   } else {
     const int grid = static_cast<int>(std::min<int64_t>(rows, 148 * 8));
     chitu::layernorm_affine_kernel<<<grid, chitu::kLnThreads, 0, st>>>(p);
@@ -1154,9 +1181,33 @@ int chitu_b200_gate_residual(void* x, int x_dtype, const void* y, int y_dtype, i
   p.rows_per_batch = rows_per_batch;
   p.C = C;
   p.y_fp16 = y_dtype == CHITU_DTYPE_FP16;
-  const long long total = rows * (C >> 2);
-  const int grid = grid_for(total, 256 * 4, 148 * 8);
-  chitu::gate_residual_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int64_t batches = rows / rows_per_batch;
+  // the column form wants 16-byte vectors of y, whole batches and a row that fits a block
+  if (!(C & 7) && C <= 8192 && rows % rows_per_batch == 0 && batches <= 65535 && !(reinterpret_cast<uintptr_t>(y) & 15)) {
+    const int n_vec = C >> 3;
+    const int rows_par = n_vec >= 512 ? 1 : 512 / n_vec;
+    const int threads = n_vec * rows_par;
+    const int64_t groups = (rows_per_batch + rows_par - 1) / rows_par;
+    const int64_t resident = std::max<int64_t>(1, 148 * (2048 / threads) / batches);
+    const dim3 grid(static_cast<unsigned>(std::min<int64_t>(groups, resident)), static_cast<unsigned>(batches));
+#define CHITU_GATE_Y(DT, FP16) \
+    (threads <= 512 ? chitu::gate_residual_rows_kernel<DT, FP16, 512><<<grid, threads, 0, st>>>(p, rows_par) \
+                    : chitu::gate_residual_rows_kernel<DT, FP16, 1024><<<grid, threads, 0, st>>>(p, rows_par))
+#define CHITU_GATE(DT) (p.y_fp16 ? CHITU_GATE_Y(DT, true) : CHITU_GATE_Y(DT, false))
+    if (x_dtype == CHITU_DTYPE_BF16)
+      CHITU_GATE(0);
+    else if (x_dtype == CHITU_DTYPE_FP16)
+      CHITU_GATE(1);
+    else
+      CHITU_GATE(2);
+#undef CHITU_GATE
+#undef CHITU_GATE_Y
+  } else {
+    const long long total = rows * (C >> 2);
+    const int grid = grid_for(total, 256 * 4, 148 * 8);
+    chitu::gate_residual_kernel<<<grid, 256, 0, st>>>(p);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "gate_residual: launch");
   return CHITU_OK;

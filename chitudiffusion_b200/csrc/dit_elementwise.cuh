@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "elementwise.cuh"
+
 namespace chitu {
 
 constexpr int kLnThreads = 256;
@@ -138,11 +140,6 @@ layernorm_affine_kernel(const LayerNormParams p) {
   }
 }
 
-// Warp-per-row form for rows of at most 8 KiB (Flux: 3072 bf16 channels, Wan-1.3B: 1536 fp32): the row
-// sits in registers as raw 16-byte vectors (up to 16 per lane, all loads in flight at once), the two
-// reductions are warp shuffles, and nothing waits at a block barrier.  Lane l owns vectors l, l + 32, ...
-constexpr int kLnWarpMaxVec = 16;
-
 template <int kXDtype>
 __device__ __forceinline__ void ln_unpack(const uint4 raw, float (&f)[8]) {
   // 16 bytes of the stream: 8 values when 16-bit, 4 when fp32 (f[4..7] unused)
@@ -166,82 +163,120 @@ __device__ __forceinline__ void ln_unpack(const uint4 raw, float (&f)[8]) {
   }
 }
 
-template <int kXDtype>
-__global__ void __launch_bounds__(256) layernorm_affine_warp_kernel(const LayerNormParams p) {
+// 16-bit pairs of the output type
+__device__ __forceinline__ uint32_t ln_pack(float lo, float hi, int fp16) {
+  if (fp16) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// Column form: thread t of a CTA owns the 16-byte vectors t, t + blockDim.x, ... (kVec of them) of every row the CTA
+// visits, so mul and add sit in registers (as 24 KB of loads per row they were four times the stream itself), and
+// kRows rows go through the two block reductions (mean, then the centred sum of squares) together, with the
+// next kRows in flight.  blockIdx.y is the batch.  HBM bound; us at 4096 / 6889 x 3072 bf16, 32760 x 1536 and 2000 x 5120
+// fp32 (cold L2, 6 us of launch and event included): 24.6, 31.6, 65.5, 33.8 with a warp (5120: a block) per row, so
+// 18.5, 24.6, 65.4, 22.6.
+// Up to 384 threads run two (fp32, whose rows hold half as many channels per thread: three) CTAs per SM, wider rows
+// with 64 registers and half as many rows in flight.
+template <int kXDtype, int kVec, int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads, kMaxThreads > 384 ? 1 : kXDtype == 2 ? 3 : 2) layernorm_affine_rows_kernel(const LayerNormParams p) {
+  constexpr int kLnRows = kMaxThreads <= 384 ? 4 : 2;
   constexpr int kPer = kXDtype == 2 ? 4 : 8;  // channels per 16-byte vector
-  const int lane = threadIdx.x & 31;
-  const int n_vec = p.C / kPer;               // vectors per row (a multiple of 32: checked by the host)
-  const int per_lane = n_vec >> 5;
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  __shared__ float red[2][kLnRows][32];
+  const int n_vec = p.C / kPer;
+  const int n_warps = blockDim.x >> 5;
   const float inv_c = 1.0f / static_cast<float>(p.C);
-  const float one = p.add_one ? 1.f : 0.f;
-  for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < p.rows;
-       row += warps) {
-    const uint4* src = reinterpret_cast<const uint4*>(p.x) + static_cast<size_t>(row) * n_vec;
-    uint4 raw[kLnWarpMaxVec];
+  const long long batch = blockIdx.y;
+  const long long row_end = p.rows_per_batch;
+  const uint4* x = static_cast<const uint4*>(p.x) + batch * p.rows_per_batch * n_vec;
+  uint16_t* out = static_cast<uint16_t*>(p.out) + batch * p.rows_per_batch * p.C;
+
+  float m[kVec][kPer], a[kVec][kPer];
 #pragma unroll
-    for (int i = 0; i < kLnWarpMaxVec; ++i)
-      if (i < per_lane) raw[i] = __ldcs(src + lane + i * 32);
-    float sum = 0.f;
+  for (int v = 0; v < kVec; ++v) {
+    const int vec = threadIdx.x + v * blockDim.x;
 #pragma unroll
-    for (int i = 0; i < kLnWarpMaxVec; ++i)
-      if (i < per_lane) {
-        float f[8];
-        ln_unpack<kXDtype>(raw[i], f);
-#pragma unroll
-        for (int e = 0; e < kPer; ++e) sum += f[e];
+    for (int e = 0; e < kPer; e += 4) {
+      float4 mv = make_float4(1.f, 1.f, 1.f, 1.f), av = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (vec < n_vec && p.mul) {
+        mv = __ldg(reinterpret_cast<const float4*>(p.mul + batch * p.mul_batch_stride + vec * kPer + e));
+        if (p.add_one) { mv.x += 1.f; mv.y += 1.f; mv.z += 1.f; mv.w += 1.f; }
       }
+      if (vec < n_vec && p.add)
+        av = __ldg(reinterpret_cast<const float4*>(p.add + batch * p.add_batch_stride + vec * kPer + e));
+      m[v][e] = mv.x; m[v][e + 1] = mv.y; m[v][e + 2] = mv.z; m[v][e + 3] = mv.w;
+      a[v][e] = av.x; a[v][e + 1] = av.y; a[v][e + 2] = av.z; a[v][e + 3] = av.w;
+    }
+  }
+  const long long step = static_cast<long long>(gridDim.x) * kLnRows;
+  long long row = static_cast<long long>(blockIdx.x) * kLnRows;
+  uint4 cur[kLnRows][kVec], nxt[kLnRows][kVec];
+  auto load = [&](uint4 (&buf)[kLnRows][kVec], long long row0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float mean = sum * inv_c;
-    float sq = 0.f;
+    for (int r = 0; r < kLnRows; ++r)
 #pragma unroll
-    for (int i = 0; i < kLnWarpMaxVec; ++i)
-      if (i < per_lane) {
-        float f[8];
-        ln_unpack<kXDtype>(raw[i], f);
-#pragma unroll
-        for (int e = 0; e < kPer; ++e) sq = fmaf(f[e] - mean, f[e] - mean, sq);
+      for (int v = 0; v < kVec; ++v) {
+        const int vec = threadIdx.x + v * blockDim.x;
+        buf[r][v] = make_uint4(0u, 0u, 0u, 0u);
+        if (vec < n_vec && row0 + r < row_end) buf[r][v] = __ldcs(x + (row0 + r) * n_vec + vec);
       }
+  };
+  load(cur, row);
+  for (; row < row_end; row += step) {
+    load(nxt, row + step);
+    float s[kLnRows], mean[kLnRows];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    const float rstd = rsqrtf(sq * inv_c + p.eps);
-    const long long b = row / p.rows_per_batch;
-    const float* mul = p.mul ? p.mul + b * p.mul_batch_stride : nullptr;
-    const float* add = p.add ? p.add + b * p.add_batch_stride : nullptr;
-    uint16_t* dst = static_cast<uint16_t*>(p.out) + static_cast<size_t>(row) * p.C;
+    for (int r = 0; r < kLnRows; ++r) {
+      s[r] = 0.f;
 #pragma unroll
-    for (int i = 0; i < kLnWarpMaxVec; ++i)
-      if (i < per_lane) {
-        const int c0 = (lane + i * 32) * kPer;
-        float f[8], r[8];
-        ln_unpack<kXDtype>(raw[i], f);
+      for (int v = 0; v < kVec; ++v) {
+        float f[8];
+        ln_unpack<kXDtype>(cur[r][v], f);
 #pragma unroll
-        for (int q = 0; q < kPer; q += 4) {
-          float4 m = mul ? __ldg(reinterpret_cast<const float4*>(mul + c0 + q)) : make_float4(1.f, 1.f, 1.f, 1.f);
-          const float4 a = add ? __ldg(reinterpret_cast<const float4*>(add + c0 + q)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (mul) { m.x += one; m.y += one; m.z += one; m.w += one; }
-          r[q] = fmaf((f[q] - mean) * rstd, m.x, a.x);
-          r[q + 1] = fmaf((f[q + 1] - mean) * rstd, m.y, a.y);
-          r[q + 2] = fmaf((f[q + 2] - mean) * rstd, m.z, a.z);
-          r[q + 3] = fmaf((f[q + 3] - mean) * rstd, m.w, a.w);
-        }
-        uint32_t o[4];
+        for (int e = 0; e < kPer; ++e) s[r] += f[e];
+      }
+    }
+    block_sums<kLnRows>(s, red[0], n_warps);
 #pragma unroll
-        for (int q = 0; q < kPer / 2; ++q) {
-          if (p.out_fp16) {
-            const __half2 h = __floats2half2_rn(r[2 * q], r[2 * q + 1]);
-            o[q] = *reinterpret_cast<const uint32_t*>(&h);
-          } else {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(r[2 * q], r[2 * q + 1]);
-            o[q] = *reinterpret_cast<const uint32_t*>(&h);
-          }
-        }
+    for (int r = 0; r < kLnRows; ++r) {
+      mean[r] = s[r] * inv_c;
+      s[r] = 0.f;
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) {
+        if (static_cast<int>(threadIdx.x + v * blockDim.x) >= n_vec) continue;
+        float f[8];
+        ln_unpack<kXDtype>(cur[r][v], f);
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) s[r] = fmaf(f[e] - mean[r], f[e] - mean[r], s[r]);
+      }
+    }
+    block_sums<kLnRows>(s, red[1], n_warps);
+#pragma unroll
+    for (int r = 0; r < kLnRows; ++r) {
+      const float rstd = rsqrtf(s[r] * inv_c + p.eps);
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) {
+        const int vec = threadIdx.x + v * blockDim.x;
+        if (vec >= n_vec || row + r >= row_end) continue;
+        float f[8], y[kPer];
+        ln_unpack<kXDtype>(cur[r][v], f);
+#pragma unroll
+        for (int e = 0; e < kPer; ++e) y[e] = fmaf((f[e] - mean[r]) * rstd, m[v][e], a[v][e]);
+        uint16_t* dst = out + (row + r) * p.C + vec * kPer;
         if constexpr (kPer == 8)
-          *reinterpret_cast<uint4*>(dst + c0) = make_uint4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<uint4*>(dst) = make_uint4(ln_pack(y[0], y[1], p.out_fp16), ln_pack(y[2], y[3], p.out_fp16),
+                                                      ln_pack(y[4], y[5], p.out_fp16), ln_pack(y[6], y[7], p.out_fp16));
         else
-          *reinterpret_cast<uint2*>(dst + c0) = make_uint2(o[0], o[1]);
+          *reinterpret_cast<uint2*>(dst) = make_uint2(ln_pack(y[0], y[1], p.out_fp16), ln_pack(y[2], y[3], p.out_fp16));
       }
+    }
+#pragma unroll
+    for (int r = 0; r < kLnRows; ++r)
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) cur[r][v] = nxt[r][v];
   }
 }
 
@@ -281,6 +316,69 @@ gate_residual_kernel(const GateResidualParams p) {
     xv.z = fmaf(y1.x, g.z, xv.z);
     xv.w = fmaf(y1.y, g.w, xv.w);
     stream_st4(p.x, p.x_dtype, static_cast<size_t>(i), xv);
+  }
+}
+
+// Column form of the same update: a thread owns eight channels (its gate sits in registers) of every row its CTA
+// visits, four rows in flight.  The CTA's threads are rows_par rows side by side, blockIdx.y is the batch.  (The
+// general kernel divides 64-bit indices for every 4 elements and reads the gate each time.)  HBM bound; us at
+// 4096 / 6889 x 3072 bf16 and 32760 x 1536 fp32 (cold L2, 6 us of launch and event included): 35.7, 55.3, 109.5 ->
+// 20.5, 28.7, 86.1.
+template <int kXDtype, bool kYFp16, int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads) gate_residual_rows_kernel(const GateResidualParams p, int rows_par) {
+  constexpr int kGateRows = kMaxThreads <= 512 ? 4 : 2;
+  const int n_vec = p.C >> 3;
+  const int sub = threadIdx.x / n_vec;
+  const int vec = threadIdx.x - sub * n_vec;
+  const long long batch = blockIdx.y;
+  float g[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) g[e] = 1.f;
+  if (p.gate) {
+    const float4* gp = reinterpret_cast<const float4*>(p.gate + batch * p.gate_batch_stride) + vec * 2;
+    const float4 g0 = __ldg(gp), g1 = __ldg(gp + 1);
+    g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w;
+    g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
+  }
+  constexpr int kXVecs = kXDtype == 2 ? 2 : 1;  // 16-byte vectors of eight stream channels
+  uint4* x = static_cast<uint4*>(p.x) + (batch * p.rows_per_batch * n_vec + vec) * kXVecs;
+  const uint4* y = static_cast<const uint4*>(p.y) + batch * p.rows_per_batch * n_vec + vec;
+  const long long step = static_cast<long long>(gridDim.x) * rows_par;
+  for (long long row0 = static_cast<long long>(blockIdx.x) * rows_par + sub; row0 < p.rows_per_batch; row0 += step * kGateRows) {
+    uint4 yv[kGateRows], xv[kGateRows][kXVecs];
+#pragma unroll
+    for (int r = 0; r < kGateRows; ++r) {
+      const long long row = row0 + r * step;
+      if (row < p.rows_per_batch) {
+        yv[r] = __ldcs(y + row * n_vec);
+#pragma unroll
+        for (int i = 0; i < kXVecs; ++i) xv[r][i] = __ldcs(x + row * n_vec * kXVecs + i);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kGateRows; ++r) {
+      const long long row = row0 + r * step;
+      if (row >= p.rows_per_batch) continue;
+      float fy[8], fx[8];
+      ln_unpack<kYFp16 ? 1 : 0>(yv[r], fy);
+      if constexpr (kXDtype == 2) {
+        const uint4 lo = xv[r][0], hi = xv[r][1];
+        fx[0] = __uint_as_float(lo.x); fx[1] = __uint_as_float(lo.y); fx[2] = __uint_as_float(lo.z); fx[3] = __uint_as_float(lo.w);
+        fx[4] = __uint_as_float(hi.x); fx[5] = __uint_as_float(hi.y); fx[6] = __uint_as_float(hi.z); fx[7] = __uint_as_float(hi.w);
+      } else {
+        ln_unpack<kXDtype>(xv[r][0], fx);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) fx[e] = fmaf(fy[e], g[e], fx[e]);
+      uint4* dst = x + row * n_vec * kXVecs;
+      if constexpr (kXDtype == 2) {
+        dst[0] = make_uint4(__float_as_uint(fx[0]), __float_as_uint(fx[1]), __float_as_uint(fx[2]), __float_as_uint(fx[3]));
+        dst[1] = make_uint4(__float_as_uint(fx[4]), __float_as_uint(fx[5]), __float_as_uint(fx[6]), __float_as_uint(fx[7]));
+      } else {
+        dst[0] = make_uint4(ln_pack(fx[0], fx[1], kXDtype), ln_pack(fx[2], fx[3], kXDtype), ln_pack(fx[4], fx[5], kXDtype),
+                            ln_pack(fx[6], fx[7], kXDtype));
+      }
+    }
   }
 }
 

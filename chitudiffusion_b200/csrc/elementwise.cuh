@@ -60,6 +60,37 @@ __device__ __forceinline__ void st4(void* p, int dtype, size_t i, float4 v) {
   }
 }
 
+// Sums of kRows values (2 or 4) over the block, in every thread; one barrier.  red[kRows][32] must not be in use by an
+// earlier call that a thread of the block may still be in (two buffers in turn are enough).  The rows are folded into
+// each other on the way through the warp - 13 shuffles for four rows instead of 40.
+template <int kRows>
+__device__ __forceinline__ void block_sums(float (&s)[kRows], float (*red)[32], int n_warps) {
+  static_assert(kRows == 2 || kRows == 4, "rows that fold into a warp");
+  constexpr int kGroup = 32 / kRows;  // lanes per row once folded
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool hi = lane & 16;
+  float v;
+  if constexpr (kRows == 4) {
+    const float a = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16);
+    const float b = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
+    const bool odd = lane & 8;
+    v = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+  } else {
+    v = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 16);
+  }
+#pragma unroll
+  for (int o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  const int row = lane / kGroup, l = lane % kGroup;
+  if (l == 0) red[row][warp] = v;
+  __syncthreads();
+  v = 0.f;
+  for (int w = l; w < n_warps; w += kGroup) v += red[row][w];
+#pragma unroll
+  for (int o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) s[r] = __shfl_sync(0xffffffffu, v, r * kGroup);
+}
+
 // ----------------------------------------------------------------------------
 // LSE combine: one warp per (b, s, h) row of D values.
 // ----------------------------------------------------------------------------
@@ -101,6 +132,72 @@ lse_combine_kernel(float* __restrict__ acc_out, float* __restrict__ acc_lse, con
       if (final_out != nullptr) st4(final_out, final_dtype, base + d, r);
     }
     if (lane == 0) acc_lse[row] = new_lse;
+  }
+}
+
+// The same for 16-bit blocks of head_dim 128 (what ring attention folds): half a warp per row, eight channels per
+// lane, four rows of a warp in flight, 32-bit indices.  The weights are the general kernel's, bit for bit.
+// HBM bound (bytes per element: 4 + 2 read, 4 written); us at 8190 x 12 heads (cold L2, 6 us of
+// launch and event included): first block 28.7 -> 20.5, further ones 38.0 -> 26.7.
+constexpr int kCombineRows = 4;
+
+template <bool kFp16, bool kFirst>
+__global__ void __launch_bounds__(256)
+lse_combine_d128_kernel(float* __restrict__ acc_out, float* __restrict__ acc_lse, const void* __restrict__ blk_out,
+                        const float* __restrict__ blk_lse, int S, int H, int rows) {
+  const int lane = threadIdx.x & 31;
+  const int half = lane >> 4, l16 = lane & 15;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int group = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); group * kCombineRows < rows; group += warps) {
+    uint4 ob[2];
+    float4 oa[2][2];
+    float lb[2], la[2];
+    int row[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      row[i] = min(group * kCombineRows + 2 * i + half, rows - 1);
+      const size_t base = static_cast<size_t>(row[i]) * 128 + l16 * 8;
+      ob[i] = __ldcs(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(blk_out) + base));
+      const int bs = row[i] / H, h = row[i] - bs * H;
+      const int b = bs / S, s = bs - b * S;
+      lb[i] = __ldg(blk_lse + static_cast<size_t>(b * H + h) * S + s);
+      if constexpr (!kFirst) {
+        oa[i][0] = *reinterpret_cast<const float4*>(acc_out + base);
+        oa[i][1] = *reinterpret_cast<const float4*>(acc_out + base + 4);
+        la[i] = acc_lse[row[i]];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (group * kCombineRows + 2 * i + half >= rows) continue;
+      float f[8];
+      const uint32_t w4[4] = {ob[i].x, ob[i].y, ob[i].z, ob[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if constexpr (kFp16) {
+          const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w4[e]));
+          f[2 * e] = v.x;
+          f[2 * e + 1] = v.y;
+        } else {
+          f[2 * e] = __uint_as_float(w4[e] << 16);
+          f[2 * e + 1] = __uint_as_float(w4[e] & 0xffff0000u);
+        }
+      }
+      float new_lse = lb[i];
+      if constexpr (!kFirst) {
+        const float x = lb[i] - la[i];  // weight of the block = sigmoid(lse_b - lse)
+        const float w = 1.0f / (1.0f + expf(-x));
+        const float y = -x;
+        new_lse = la[i] - (fminf(y, 0.f) - log1pf(expf(-fabsf(y))));
+        const float a8[8] = {oa[i][0].x, oa[i][0].y, oa[i][0].z, oa[i][0].w, oa[i][1].x, oa[i][1].y, oa[i][1].z, oa[i][1].w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = a8[e] - w * (a8[e] - f[e]);
+      }
+      float4* dst = reinterpret_cast<float4*>(acc_out + static_cast<size_t>(row[i]) * 128 + l16 * 8);
+      dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+      dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+      if (l16 == 0) acc_lse[row[i]] = new_lse;
+    }
   }
 }
 
@@ -210,7 +307,7 @@ struct NormRopeTokens {
 // NormRopeParams, kRound 0 (no intermediate rounding), 1 (round the normalised value to the input
 // type, as `type_as(x)` does) or 2 (also round after the weight multiply), kOutBf16 the store type.
 template <int kInDtype, int kNormMode, int kRopeMode, int kRound, bool kOutBf16>
-__device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float (*red)[NormRopeTokens<kInDtype>::value][kNormMaxThreads / 32]) {
+__device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float (*red)[NormRopeTokens<kInDtype>::value][32]) {
   constexpr int kTok = NormRopeTokens<kInDtype>::value;
   constexpr int kOutDtype = kOutBf16 ? kBF16 : kFP16;
   const int C = p.H * p.D;
@@ -269,20 +366,11 @@ __device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float 
         float ss = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if ((threadIdx.x & 31) == 0) red[phase][i][threadIdx.x >> 5] = ss;
+        rstd_full[i] = ss;
       }
-      __syncthreads();  // red[phase] is rewritten two iterations later, after the next barrier
-      // every warp sums the per-warp partials itself: one shared-memory read per lane, then shuffles
+      block_sums<kTok>(rstd_full, red[phase], n_warps);  // red[phase] is rewritten two iterations later
 #pragma unroll
-      for (int i = 0; i < kTok; ++i) {
-        const int lane = threadIdx.x & 31;
-        float tot = lane < n_warps ? red[phase][i][lane] : 0.f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-        rstd_full[i] = rsqrtf(tot * inv_n + p.eps);
-      }
+      for (int i = 0; i < kTok; ++i) rstd_full[i] = rsqrtf(rstd_full[i] * inv_n + p.eps);
     }
 
     // batch and position of the first token of the iteration; the others follow by increments
@@ -413,7 +501,7 @@ __device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float 
 // cast / scatter whatever the launch's template modes are.
 template <int kInDtype, int kNormModeT, int kRopeModeT>
 __device__ __forceinline__ void qk_norm_rope_dispatch(const NormRopeBatch& batch,
-                                                      float (*red)[NormRopeTokens<kInDtype>::value][kNormMaxThreads / 32]) {
+                                                      float (*red)[NormRopeTokens<kInDtype>::value][32]) {
   const NormRopeParams& p = batch.job[blockIdx.y];
   const bool out_bf16 = p.out_dtype == kBF16;
   if (p.norm_mode == 2 && p.rope_mode == 0) {
@@ -442,7 +530,7 @@ __device__ __forceinline__ void qk_norm_rope_dispatch(const NormRopeBatch& batch
 // ends by publishing "my rows have landed" to every peer (last-block pattern).
 template <int kInDtype, int kNormModeT, int kRopeModeT>
 __device__ __forceinline__ void qk_norm_rope_body(const NormRopeBatch& batch) {
-  __shared__ float red[2][NormRopeTokens<kInDtype>::value][kNormMaxThreads / 32];
+  __shared__ float red[2][NormRopeTokens<kInDtype>::value][32];
   qk_norm_rope_dispatch<kInDtype, kNormModeT, kRopeModeT>(batch, red);
   if (batch.signal) {
     __syncthreads();
