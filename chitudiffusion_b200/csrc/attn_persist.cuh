@@ -18,8 +18,17 @@
 // have not started yet (clusterlaunchcontrol), one ahead of what it is working on.  So there is no counter
 // in memory to reset, and an SM that another kernel holds (a collective on a side stream) simply takes none.
 //
-// Roles and tensor memory as in attn_fwd_kernel.  Between two query blocks of a CTA:
-//   * Q_t is free once the last QK^T of tile t has run, S_t once the last PV has consumed P_t (issue order);
+// Tensor memory (512 columns): S | P0 | P1 | O0 | O1 with ONE set of 128 score columns for both query tiles, and
+// probabilities of their own (64 columns each) instead of over their scores.  A tile's scores leave for registers
+// in some 150 cycles, so the next QK^T - the other tile's - starts there while the exponentials are formed, and no
+// tile waits for PV and QK^T of its own between two steps (in attn_fwd_kernel 1030 of every 2850 cycles).
+//
+// Warps: 0-3 / 4-7 softmax of tile 0 / 1, 8 issues QK^T of both tiles in turn, 9 TMA, 10 / 11 issue PV of tile
+// 0 / 1.  With one issuing thread (its six waits per step each let the tensor pipe run dry) the same layout took
+// 218 us at S = 4608, H = 24, with three 195; S and P of a tile overlaid, as in attn_fwd_kernel, 201.
+//
+// Between two query blocks of a CTA:
+//   * Q_t is free once the last QK^T of tile t has run;
 //   * O_t is overwritten by the next block's first PV, which waits for probabilities that the same
 //     softmax warps form after their epilogue has read O_t.
 #pragma once
@@ -103,6 +112,111 @@ struct Ring {
   }
 };
 
+// Where a softmax warp's query tile lives: tensor-memory addresses (this warp's lanes) and barriers.
+struct TileRefs {
+  uint32_t t_s, t_p, t_o;  // scores (both tiles share them), this tile's probabilities and accumulator
+  uint32_t bar_s_empty;    // the scores are in registers (one arrival per warp)
+  uint32_t bar_p;          // [2] keys [0, 64) and [64, 128) of the probabilities are stored (every thread arrives)
+  uint32_t bar_pv;         // a step's PV is complete (phase = step)
+};
+
+// One softmax step of a query tile's four warps (thread = one row, 128 scores): scores in, probabilities out.
+// `step` counts the tile's steps since the launch, `first` says that there is no accumulator yet, `valid` how many keys
+// of the tile exist (kTileN: all).
+//
+// The scores go to registers at once and their tensor memory is given back before anything else, because the
+// other tile's scores are computed into the same columns meanwhile.  Every exponential takes the MUFU unit: 128 of them
+// are 1024 of its cycles, two warps' worth what the tensor pipe needs for a step of both tiles, and now that no
+// chain holds the warps up the polynomial of attn_fwd_kernel only costs issue slots (of every 8 pairs 2 / 1 / 0
+// polynomial: 203 / 195 / 195 us at S = 4608, H = 24, 4768 / 4678 / 4665 us at S = 32760, H = 12).
+template <bool kFp16>
+__device__ __forceinline__ void persist_softmax_step(const TileRefs& r, int step, bool first, int valid, float sl2,
+                                                     float& m_used, float& l_sum, volatile int* abort_flag, int* status) {
+  uint32_t s[4][32];
+  float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld32(r.t_s + c * 32, s[c]);
+  tmem_wait_ld();
+  tc_fence_before_sync();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(r.bar_s_empty);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (valid < kTileN) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (c * 32 + i >= valid) s[c][i] = 0xff800000u;  // -inf
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      mx0 = max3(mx0, __uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1]));
+      mx1 = max3(mx1, __uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3]));
+    }
+  }
+  const float mx = fmaxf(mx0, mx1);
+
+  if (first) {
+    m_used = mx;
+  } else {
+    const bool need = (mx - m_used) * sl2 > kRescaleThreshold;
+    if (__any_sync(0xffffffffu, need)) {
+      mbar_wait(r.bar_pv, (step - 1) & 1, abort_flag, status, kDevTimeoutSoftmax);
+      tc_fence_after_sync();
+      const float f = need ? fast_exp2((m_used - mx) * sl2) : 1.0f;
+#pragma unroll 1
+      for (int c = 0; c < 8; ++c) {
+        uint32_t o[16];
+        tmem_ld16(r.t_o + c * 16, o);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+        tmem_st16(r.t_o + c * 16, o);
+      }
+      l_sum *= f;
+      if (need) m_used = mx;
+    }
+  }
+
+  // (looked at early, so that the answer is there when the first probabilities are stored)
+  const bool pv_done = step == 0 || mbar_try_wait(r.bar_pv, (step - 1) & 1);
+
+  // p = 2^(s*scale - m*scale): packed two-wide FMA / add, one MUFU per element
+  const float2 sl2_2 = make_float2(sl2, sl2);
+  // (a row without a finite score so far has nothing to subtract: its probabilities are zero, not NaN)
+  const float neg_m = m_used == -INFINITY ? 0.f : -m_used * sl2;
+  const float2 neg_m2 = make_float2(neg_m, neg_m);
+  uint32_t pk[2][32];
+  float2 la = make_float2(0.f, 0.f), lb = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      float2 x0 = __ffma2_rn(make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sl2_2, neg_m2);
+      float2 x1 =
+          __ffma2_rn(make_float2(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3])), sl2_2, neg_m2);
+      x0.x = fast_exp2(x0.x);
+      x0.y = fast_exp2(x0.y);
+      x1.x = fast_exp2(x1.x);
+      x1.y = fast_exp2(x1.y);
+      la = __fadd2_rn(la, x0);
+      lb = __fadd2_rn(lb, x1);
+      pk[c >> 1][(c & 1) * 16 + (i >> 1)] = pack2<kFp16>(x0.x, x0.y);
+      pk[c >> 1][(c & 1) * 16 + (i >> 1) + 1] = pack2<kFp16>(x1.x, x1.y);
+      if ((c & 1) == 1 && i == 28) {
+        // 64 probabilities done: hand this half to the MMA warp
+        if (c == 1) {
+          if (!pv_done) mbar_wait(r.bar_pv, (step - 1) & 1, abort_flag, status, kDevTimeoutSoftmax);
+          tc_fence_after_sync();
+        }
+        tmem_st32(r.t_p + (c >> 1) * 32, pk[c >> 1]);
+        tmem_wait_st();
+        tc_fence_before_sync();
+        mbar_arrive(r.bar_p + 8 * (c >> 1));
+      }
+    }
+  l_sum += (la.x + la.y) + (lb.x + lb.y);
+}
+
 // The steps of a unit, one run of one query block's key tiles at a time.
 struct UnitWalk {
   int pos, end;
@@ -148,9 +262,10 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   const uint32_t bar_kv_empty = bar_kv_full + 8 * kSt;         // [kSt]
   const uint32_t bar_s_full = bar_kv_empty + 8 * kSt;          // [2]
   const uint32_t bar_p_full = bar_s_full + 16;                 // [2][2]
-  const uint32_t bar_o_final = bar_p_full + 32;                // [2]
-  const uint32_t bar_drain = bar_o_final + 16;
-  uint8_t* tail = ctl_gen + (16 + 8 + 8) * kClcStages + 32 + 16 * kSt + 16 + 32 + 16 + 8;
+  const uint32_t bar_pv = bar_p_full + 32;                     // [2]
+  const uint32_t bar_s_empty = bar_pv + 16;
+  const uint32_t bar_drain = bar_s_empty + 8;                  // [3]
+  uint8_t* tail = ctl_gen + (16 + 8 + 8) * kClcStages + 32 + 16 * kSt + 16 + 32 + 16 + 8 + 24;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
   volatile int* merge_flag = reinterpret_cast<volatile int*>(tail + 16);  // [2 tiles]
@@ -162,11 +277,11 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
     *abort_flag = 0;
     for (int s = 0; s < kClcStages; ++s) {
       mbar_init(bar_clc_full + 8 * s, 1);
-      mbar_init(bar_clc_empty + 8 * s, 9);  // the MMA warp and the eight softmax warps
+      mbar_init(bar_clc_empty + 8 * s, 11);  // the three MMA warps and the eight softmax warps
     }
     for (int s = 0; s < kSt; ++s) {
       mbar_init(bar_kv_full + 8 * s, 1);
-      mbar_init(bar_kv_empty + 8 * s, 1);
+      mbar_init(bar_kv_empty + 8 * s, 1 + (s & 1));  // keys (even slots): one reader; values (odd slots): two
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(bar_q_full + 8 * t, 1);
@@ -174,9 +289,10 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       mbar_init(bar_s_full + 8 * t, 1);
       mbar_init(bar_p_full + 16 * t, kTileM);
       mbar_init(bar_p_full + 16 * t + 8, kTileM);
-      mbar_init(bar_o_final + 8 * t, 1);
+      mbar_init(bar_pv + 8 * t, 1);
     }
-    mbar_init(bar_drain, 1);
+    mbar_init(bar_s_empty, 4);
+    for (int i = 0; i < 3; ++i) mbar_init(bar_drain + 8 * i, 1);
     mbar_fence_init();
   }
   if (warp == 8) {
@@ -220,7 +336,7 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   };
 
   if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     if (warp == 9) {
       // ---------------------------------------------------------------- TMA producer; asks for the next unit
       int n_units = 0;
@@ -294,122 +410,131 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(bar_kv_full + 8 * i, i < ring.slot ? ring.phase : ring.phase ^ 1); ++spin) {
           }
       }
-    } else if (warp == 8) {
-      // ---------------------------------------------------------------- MMA issuer
-      constexpr uint32_t kIdescQK = umma_idesc(1, kFp16 ? 0 : 1, kFp16 ? 0 : 1, 0, kTileM, kTileN);
-      constexpr uint32_t kIdescPV = umma_idesc(1, kFp16 ? 0 : 1, kFp16 ? 0 : 1, 1, kTileM, kHeadDim);
+    } else {
+      // ---------------------------------------------------------------- MMA issuers
+      // Warp 8 issues every QK^T, warps 10 and 11 the PV of tile 0 and 1.  An issuing thread is held up while the
+      // tensor pipe works off what it has issued, and a wait costs it some 100 cycles even when there is nothing to
+      // wait for: with one thread for all three kinds the pipe ran dry at each of its six waits per step.
       const bool leader = elect_one();
-      const uint64_t q_desc0 = umma_smem_desc_sw128(q_smem, 16, 1024);
-      const uint64_t k_desc0 = umma_smem_desc_sw128(kv_smem, 16, 1024);
-      const uint64_t v_desc0 = umma_smem_desc_sw128(kv_smem, kHalfTileBytes, 1024);
-      auto issue_qk = [&](int t, int slot) {
-        const uint64_t a0 = q_desc0 + static_cast<uint64_t>((t * kTileBytes) >> 4);
-        const uint64_t b0 = k_desc0 + static_cast<uint64_t>((slot * kTileBytes) >> 4);
-        const uint32_t d = tmem_base + t * kTileN;
-#pragma unroll
-        for (int k = 0; k < kHeadDim / 16; ++k) {
-          const uint64_t off = static_cast<uint64_t>(((k >> 2) * kHalfTileBytes + (k & 3) * 32) >> 4);
-          umma_ss_f16(d, a0 + off, b0 + off, kIdescQK, k > 0);
-        }
-      };
-      auto issue_pv_half = [&](int t, int slot, int h, bool accumulate) {
-        const uint64_t b0 = v_desc0 + static_cast<uint64_t>((slot * kTileBytes + h * 8192) >> 4);
-        const uint32_t d = tmem_base + 2 * kTileN + t * kHeadDim;
-        const uint32_t a = tmem_base + t * kTileN + h * 32;
-        const uint32_t acc0 = accumulate ? 1u : 0u;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          umma_ts_f16(d, a + k * 8, b0 + static_cast<uint64_t>((k * 2048) >> 4), kIdescPV, k > 0 ? 1u : acc0);
-        }
-      };
+      const int role = warp == 8 ? 0 : warp - 9;  // 0 scores; 1, 2 PV of tile 0, 1
       int n_units = 0;
-      Ring ring;               // the next K/V item to consume
-      int q_uses[2] = {0, 0};  // Q tiles consumed so far
-      int steps[2] = {0, 0};   // steps of each tile so far
-      auto wait_item = [&](const Ring& r) {
-        mbar_wait(bar_kv_full + 8 * r.slot, r.phase, abort_flag, p.status, kDevTimeoutMma);
+      Ring ring;  // the next K (scores) or V item to consume
+      if (role > 0) ring.advance();
+      auto wait_item = [&] {
+        mbar_wait(bar_kv_full + 8 * ring.slot, ring.phase, abort_flag, p.status, kDevTimeoutMma);
       };
       int unit = blockIdx.x;
-      while (unit >= 0) {
-        UnitWalk walk(p, unit);
-        int item, kv0, n;
-        while (walk.next(p, item, kv0, n)) {
-          const int n_qt = decode(item).n_qt;
-          wait_item(ring);
-          for (int t = 0; t < n_qt; ++t) {
-            mbar_wait(bar_q_full + 8 * t, q_uses[t] & 1, abort_flag, p.status, kDevTimeoutMma);
-            ++q_uses[t];
-            tc_fence_after_sync();
-            if (leader) {
-              issue_qk(t, ring.slot);
-              umma_commit(bar_s_full + 8 * t);
-              if (n == 1) umma_commit(bar_q_empty + 8 * t);
-            }
-            __syncwarp();
-          }
-          if (leader) umma_commit(bar_kv_empty + 8 * ring.slot);  // K_0 free once both QK^T have run
-          __syncwarp();
-          for (int j = 0; j < n; ++j) {
-            const bool more = j + 1 < n;
-            ring.advance();
-            const Ring iv = ring;  // V_j
-            ring.advance();
-            const Ring ik = ring;  // K_{j+1}, or the next query block's K_0
-            if (more) wait_item(ik);
-            wait_item(iv);
-            for (int t = 0; t < n_qt; ++t) {
-              // the PV MMAs of the first 64 keys start while the softmax warps still work on the rest
-              const int par = steps[t] & 1;
-              ++steps[t];
-              mbar_wait(bar_p_full + 16 * t, par, abort_flag, p.status, kDevTimeoutMma);
-              tc_fence_after_sync();
-              if (leader) issue_pv_half(t, iv.slot, 0, j > 0);
-              __syncwarp();
-              mbar_wait(bar_p_full + 16 * t + 8, par, abort_flag, p.status, kDevTimeoutMma);
-              tc_fence_after_sync();
-              if (leader) {
-                issue_pv_half(t, iv.slot, 1, true);
-                if (more) {
-                  issue_qk(t, ik.slot);
-                  umma_commit(bar_s_full + 8 * t);
-                  if (j + 2 == n) umma_commit(bar_q_empty + 8 * t);
-                } else {
-                  umma_commit(bar_o_final + 8 * t);
+      if (role == 0) {
+        constexpr uint32_t kIdescQK = umma_idesc(1, kFp16 ? 0 : 1, kFp16 ? 0 : 1, 0, kTileM, kTileN);
+        const uint64_t q_desc0 = umma_smem_desc_sw128(q_smem, 16, 1024);
+        const uint64_t k_desc0 = umma_smem_desc_sw128(kv_smem, 16, 1024);
+        int q_uses[2] = {0, 0};  // Q tiles consumed so far
+        int scores = 0;          // QK^T so far
+        while (unit >= 0) {
+          UnitWalk walk(p, unit);
+          int item, kv0, n;
+          while (walk.next(p, item, kv0, n)) {
+            const int n_qt = decode(item).n_qt;
+            for (int j = 0; j < n; ++j) {
+              wait_item();
+              for (int t = 0; t < n_qt; ++t) {
+                if (j == 0) {
+                  mbar_wait(bar_q_full + 8 * t, q_uses[t] & 1, abort_flag, p.status, kDevTimeoutMma);
+                  ++q_uses[t];
                 }
+                // the columns of the scores are free once the softmax warps have the previous ones in registers
+                if (scores > 0) mbar_wait(bar_s_empty, (scores - 1) & 1, abort_flag, p.status, kDevTimeoutMma);
+                ++scores;
+                tc_fence_after_sync();
+                if (leader) {
+                  // S = Q_t K^T : both operands K-major, 8 steps of 16 along head_dim
+                  const uint64_t a0 = q_desc0 + static_cast<uint64_t>((t * kTileBytes) >> 4);
+                  const uint64_t b0 = k_desc0 + static_cast<uint64_t>((ring.slot * kTileBytes) >> 4);
+#pragma unroll
+                  for (int k = 0; k < kHeadDim / 16; ++k) {
+                    const uint64_t off = static_cast<uint64_t>(((k >> 2) * kHalfTileBytes + (k & 3) * 32) >> 4);
+                    umma_ss_f16(tmem_base, a0 + off, b0 + off, kIdescQK, k > 0);
+                  }
+                  umma_commit(bar_s_full + 8 * t);
+                  if (j + 1 == n) umma_commit(bar_q_empty + 8 * t);
+                }
+                __syncwarp();
               }
+              if (leader) umma_commit(bar_kv_empty + 8 * ring.slot);
               __syncwarp();
+              ring.advance();
+              ring.advance();
             }
-            if (leader) {
-              umma_commit(bar_kv_empty + 8 * (iv.slot));
-              if (more) umma_commit(bar_kv_empty + 8 * (ik.slot));
-            }
-            __syncwarp();
           }
+          unit = next_unit(n_units++, kDevTimeoutMma);
+          if (*abort_flag) unit = -1;
         }
-        unit = next_unit(n_units++, kDevTimeoutMma);
-        if (*abort_flag) unit = -1;
+      } else {
+        constexpr uint32_t kIdescPV = umma_idesc(1, kFp16 ? 0 : 1, kFp16 ? 0 : 1, 1, kTileM, kHeadDim);
+        const int t = role - 1;
+        const uint64_t v_desc0 = umma_smem_desc_sw128(kv_smem, kHalfTileBytes, 1024);
+        const uint32_t t_p = tmem_base + kTileN + t * 64;
+        const uint32_t t_o = tmem_base + 2 * kTileN + t * kHeadDim;
+        int steps = 0;  // the tile's steps so far
+        while (unit >= 0) {
+          UnitWalk walk(p, unit);
+          int item, kv0, n;
+          while (walk.next(p, item, kv0, n)) {
+            const int n_qt = decode(item).n_qt;
+            for (int j = 0; j < n; ++j) {
+              wait_item();
+              if (t < n_qt) {
+                // the PV MMAs of the first 64 keys start while the softmax warps still work on the rest
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  mbar_wait(bar_p_full + 16 * t + 8 * h, steps & 1, abort_flag, p.status, kDevTimeoutMma);
+                  tc_fence_after_sync();
+                  if (leader) {
+                    // O_t += P_t[:, 64h .. 64h+64) V[64h .. 64h+64) : A = P from tensor memory (two 16-bit values
+                    // per column), B = V tile as loaded ([key][d], d contiguous => MN-major), 4 steps of 16 keys
+                    const uint64_t b0 = v_desc0 + static_cast<uint64_t>((ring.slot * kTileBytes + h * 8192) >> 4);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                      umma_ts_f16(t_o, t_p + h * 32 + k * 8, b0 + static_cast<uint64_t>((k * 2048) >> 4), kIdescPV,
+                                  (h > 0 || k > 0 || j > 0) ? 1u : 0u);
+                    if (h == 1) umma_commit(bar_pv + 8 * t);
+                  }
+                  __syncwarp();
+                }
+                ++steps;
+              }
+              if (leader) umma_commit(bar_kv_empty + 8 * ring.slot);
+              __syncwarp();
+              ring.advance();
+              ring.advance();
+            }
+          }
+          unit = next_unit(n_units++, kDevTimeoutMma);
+          if (*abort_flag) unit = -1;
+        }
       }
       // One more commit and a bounded poll on it: every arrival of this warp's commits has landed, and nothing
       // writes tensor memory after it has been freed below.
-      if (leader) umma_commit(bar_drain);
+      if (leader) umma_commit(bar_drain + 8 * role);
       __syncwarp();
-      for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(bar_drain, 0); ++spin) {
+      for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(bar_drain + 8 * role, 0); ++spin) {
       }
     }
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     const int t = warp >> 2;
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t t_s = tmem_base + lane_base + t * kTileN;
     const uint32_t t_o = tmem_base + lane_base + 2 * kTileN + t * kHeadDim;
+    const TileRefs refs{tmem_base + lane_base, tmem_base + lane_base + kTileN + t * 64, t_o, bar_s_empty, bar_p_full + 16 * t,
+                        bar_pv + 8 * t};
     uint8_t* stage = store_smem + warp * 4096;
     const float sl2 = p.scale_log2;
     const int tail_valid = p.Sk - (p.n_kv - 1) * kTileN;  // 1..128 valid keys in the last tile of K
     int n_units = 0;
-    int steps = 0, finals = 0;  // this tile's steps and finished query blocks so far
+    int steps = 0;  // this tile's steps so far
     constexpr int kNotAsked = -2;
     int unit = blockIdx.x;
     while (unit >= 0) {
@@ -424,13 +549,12 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         for (int j = 0; j < n; ++j, ++steps) {
           mbar_wait(bar_s_full + 8 * t, steps & 1, abort_flag, p.status, kDevTimeoutSoftmax);
           tc_fence_after_sync();
-          softmax_step<kFp16>(t_s, t_o, bar_p_full + 16 * t, j == 0, kv0 + j == p.n_kv - 1 ? tail_valid : kTileN, sl2, m_used,
-                              l_sum);
+          persist_softmax_step<kFp16>(refs, steps, j == 0, kv0 + j == p.n_kv - 1 ? tail_valid : kTileN, sl2, m_used, l_sum,
+                                     abort_flag, p.status);
         }
         // (the proxy fence behind a read answer is cheap here; with the epilogue's stores in flight it took 900 cycles)
         if (walk.pos >= walk.end) following = next_unit(n_units++, kDevTimeoutSoftmax);
-        mbar_wait(bar_o_final + 8 * t, finals & 1, abort_flag, p.status, kDevTimeoutEpilogue);
-        ++finals;
+        mbar_wait(bar_pv + 8 * t, (steps - 1) & 1, abort_flag, p.status, kDevTimeoutEpilogue);
         tc_fence_after_sync();
         const bool whole = n == p.n_kv;
         // no finite score at all: undefined over a whole row, no weight in a merge

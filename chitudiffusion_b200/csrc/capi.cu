@@ -220,30 +220,25 @@ int64_t splitkv_workspace_bytes(int B, int Sq, int H, int D, int n_splits) {
 // A cut costs about kCutSteps steps (two epilogues to scratch memory instead of one to the output, and the merge).
 // Grids that do not fill the machine once are the business of the key-split entry points.
 //
-// Persistent CTAs save the five steps that a CTA of attn_fwd_kernel spends on starting and ending, but they drift
-// apart, while CTAs that start together stay together and have their reads of the same key tiles coalesced on
-// the way to L2 (S = 32760, H = 12: 460 M sectors read against 744 M, at the power limit 4.83 against 4.93 ms).
-// So long rows take the persistent kernel only where a cut gains more than that.  Measured, attn_fwd_kernel ->
-// persistent, us: 512 keys 147 -> 106 (S = 32760, H = 12); 36 key tiles 210 -> 206 (Flux, 2.9 waves);
-// 61 tiles cut 323 -> 302 (2.5 waves), 64 tiles cut 340 -> 329 (2.6 waves), uncut 340 -> 339;
-// 256 tiles cut 4835 -> 4835 (10.4 waves), uncut 4835 -> 4925.
+// The persistent kernel takes every grid that fills the machine at least once; below that a CTA has a single query
+// block and attn_fwd_kernel (whose key ranges such grids are offered) does the same work.  Measured, attn_fwd_kernel ->
+// persistent, us: 512 keys 147 -> 103 (S = 32760, H = 12); 36 key tiles 209 -> 195 (S = 4608, H = 24, 2.9 waves);
+// 61 tiles 322 -> 306, cut PERSIST_CUT (2.5 waves); 256 tiles 4850 -> 4665 (10.4 waves).
 struct CutPlan {
-  bool persistent = true;
+  bool persistent = false;
   int cut_items = 0, n_bundles = 0, bundle_steps = 1;
 };
 constexpr int kCutSteps = 5;
-constexpr int kPersistentTiles = 64;
 CutPlan plan_cut(long long items, int n_kv, int sms, bool may_cut) {
   CutPlan c;
-  c.persistent = n_kv <= kPersistentTiles;
-  if (sms <= 0 || !may_cut) return c;
+  if (sms <= 0) return c;
   const long long waves = items / sms, rem = items % sms;
-  if (waves == 0 || rem == 0) return c;
+  c.persistent = waves > 0;
+  if (waves == 0 || rem == 0 || !may_cut) return c;
   const long long per_sm = (rem * n_kv + sms - 1) / sms, floor_steps = (n_kv + 7) / 8;
   const long long steps = per_sm > floor_steps ? per_sm : floor_steps;
   const long long whole = (waves + 1) * n_kv, cut = waves * n_kv + steps + kCutSteps;
-  if (cut * 100 >= whole * (c.persistent ? 98 : 94)) return c;
-  c.persistent = true;
+  if (cut * 100 >= whole * 98) return c;
   c.cut_items = static_cast<int>(rem);
   c.bundle_steps = static_cast<int>(steps);
   c.n_bundles = static_cast<int>((rem * n_kv + steps - 1) / steps);
