@@ -12,7 +12,7 @@
 //   otherwise       one whole query block.
 // Query blocks that do not fill the last wave of the machine are cut into equal bundles, one per SM, so that
 // all SMs finish together; a bundle touches at most two query blocks and leaves a fragment of each in scratch
-// memory, and the CTA that completes a query block's last fragment merges them (nobody waits).
+// memory, and the warp that completes the last fragment of its 32 rows merges them (nobody waits).
 //
 // Units are handed out by the hardware: the grid has one CTA per unit, and a running CTA takes over units that
 // have not started yet (clusterlaunchcontrol), one ahead of what it is working on.  So there is no counter
@@ -71,7 +71,7 @@ struct AttnPersistParams {
   int n_bundles;     // bundles of
   int bundle_steps;  // key-tile steps each (<= n_kv)
   FastDiv by_n_kv, by_n_qblocks, by_batch, by_bundle_steps;
-  // scratch (cut_items > 0): counters [cut_items][2 tiles], zero between calls; a fragment's normalised fp32 rows
+  // scratch (cut_items > 0): counters [cut_items][2 tiles][4 warps], zero between calls; a fragment's normalised fp32 rows
   // [bundle * 2 + k][2 tiles][32 chunks][128 rows] float4 (k = 0, 1: the bundle's first / second query block) and
   // their natural log-sum-exps [bundle * 2 + k][2 tiles][128 rows]
   int* count;
@@ -268,7 +268,6 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   uint8_t* tail = ctl_gen + (16 + 8 + 8) * kClcStages + 32 + 16 * kSt + 16 + 32 + 16 + 8 + 24;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
-  volatile int* merge_flag = reinterpret_cast<volatile int*>(tail + 16);  // [2 tiles]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -327,13 +326,18 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   // distributor's next write into it, which goes through the async proxy).
   auto next_unit = [&](int n, int code) {
     const int st = n & (kClcStages - 1);
-    if (!mbar_wait(bar_clc_full + 8 * st, (n / kClcStages) & 1, abort_flag, p.status, code)) return -1;
+    // (lanes poll on their own and may see a wait given up at different times: the warp decides as one)
+    if (!__all_sync(0xffffffffu, mbar_wait(bar_clc_full + 8 * st, (n / kClcStages) & 1, abort_flag, p.status, code))) return -1;
     const int u = clc_unit(clc_answer + 16 * st);
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_clc_empty + 8 * st);
     return u;
   };
+
+  // A role has timed out.  Warps look on their own and may part here - one goes home, another takes up the next unit -
+  // so nothing between here and the CTA's last barrier may wait for another warp other than by a bounded mbarrier wait.
+  auto gave_up = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -387,18 +391,19 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           }
         }
         // the answer (this warp is the next to write the slot, so it needs no release)
-        if (mbar_wait(bar_clc_full + 8 * st, (n_units / kClcStages) & 1, abort_flag, p.status, kDevTimeoutLoad)) {
+        if (__all_sync(0xffffffffu, mbar_wait(bar_clc_full + 8 * st, (n_units / kClcStages) & 1, abort_flag, p.status, kDevTimeoutLoad))) {
           unit = clc_unit(clc_answer + 16 * st);
           fence_proxy_async_smem();
         } else {
           unit = -1;
         }
-        if (*abort_flag) unit = -1;
+        if (gave_up()) unit = -1;
         ++n_units;
       }
-      if (*abort_flag && lane == 0) {
-        // A role gave up: nothing of ours may still be landing in this CTA's shared memory when the CTA retires
-        // (bounded polls): the last answer, the Q tiles, the last copy into every K/V slot.
+      if (lane == 0) {
+        // Should a role give up - even after this point - nothing of ours may still be landing in this CTA's shared
+        // memory when the CTA retires (bounded polls): the last answer, the Q tiles, the last copy into every K/V slot.
+        // (Where nobody gives up, the readers wait for the same copies.)
         const int last = n_units - 1;
         for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(bar_clc_full + 8 * (last & (kClcStages - 1)), (last / kClcStages) & 1); ++spin) {
         }
@@ -467,7 +472,7 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
           }
           unit = next_unit(n_units++, kDevTimeoutMma);
-          if (*abort_flag) unit = -1;
+          if (gave_up()) unit = -1;
         }
       } else {
         constexpr uint32_t kIdescPV = umma_idesc(1, kFp16 ? 0 : 1, kFp16 ? 0 : 1, 1, kTileM, kHeadDim);
@@ -510,7 +515,7 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             }
           }
           unit = next_unit(n_units++, kDevTimeoutMma);
-          if (*abort_flag) unit = -1;
+          if (gave_up()) unit = -1;
         }
       }
       // One more commit and a bounded poll on it: every arrival of this warp's commits has landed, and nothing
@@ -589,18 +594,19 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
                               __uint_as_float(o[i + 2]) * inv_l, __uint_as_float(o[i + 3]) * inv_l);
           }
           p.part_lse[slot * kTileM + row_in_tile] = lse_row;
-          // the tile's four warps meet; one thread counts the fragment in and learns whether it is the last
-          asm volatile("bar.sync %0, %1;" ::"r"(1 + t), "r"(kTileM) : "memory");
-          if (row_in_tile == 0) {
+          // Every warp counts its 32 rows in by itself and merges them if they are the query block's last: no barrier
+          // among the tile's warps (see gave_up).
+          int done = 0;
+          __syncwarp();
+          if (lane == 0) {
             __threadfence();
-            int* counter = p.count + item * 2 + t;
-            const int done = atomicAdd(counter, 1) == last - first;
+            int* counter = p.count + (item * 2 + t) * 4 + quad;
+            done = atomicAdd(counter, 1) == last - first;
             if (done) *counter = 0;
             __threadfence();
-            merge_flag[t] = done;
           }
-          asm volatile("bar.sync %0, %1;" ::"r"(1 + t), "r"(kTileM) : "memory");
-          write_out = merge_flag[t] != 0;
+          write_out = __shfl_sync(0xffffffffu, done, 0) != 0;
+          __syncwarp();
           if (write_out) {
             // out = sum_i exp(lse_i - lse) * part_i, lse = log sum_i exp(lse_i), fragments in key order
             part0 = first;
@@ -676,7 +682,7 @@ attn_persist_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           p.lse[(static_cast<size_t>(w.batch) * p.H + w.head) * p.Sq + row] = lse_row;
       }
       unit = following == kNotAsked ? next_unit(n_units++, kDevTimeoutSoftmax) : following;
-      if (*abort_flag) unit = -1;
+      if (gave_up()) unit = -1;
     }
     if (lane == 0) tma_store_wait();
   }
