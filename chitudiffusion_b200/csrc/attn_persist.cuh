@@ -206,6 +206,7 @@ __device__ __forceinline__ void persist_softmax_step(const TileRefs& r, int step
         // 64 probabilities done: hand this half to the MMA warp
         if (c == 1) {
           if (!pv_done) mbar_wait(r.bar_pv, (step - 1) & 1, abort_flag, status, kDevTimeoutSoftmax);
+          __syncwarp();  // (lanes may have found out on their own; the store below is the warp's)
           tc_fence_after_sync();
         }
         tmem_st32(r.t_p + (c >> 1) * 32, pk[c >> 1]);

@@ -31,3 +31,10 @@ def test_a_warp_decides_as_one(code):
     assert len(re.findall(r"__any_sync\(0xffffffffu, \*abort_flag", body)) + len(re.findall(r"\*abort_flag = 0", body)) == len(uses)
     for m in re.finditer(r"(if|while)\s*\(\s*!?\s*mbar_wait", body):
         pytest.fail("control flow on one lane's wait: " + body[m.start():m.start() + 80])
+
+
+def test_lanes_meet_after_a_wait_that_only_some_take(code):
+    """Tensor-memory loads and stores are instructions of the whole warp (.sync.aligned): a wait behind a condition that a
+    lane evaluated for itself is followed by __syncwarp before the next of them."""
+    conditional = re.findall(r"if \(!pv_done\) mbar_wait\([^;]*;\s*(\S+)", code)
+    assert conditional and all(nxt.startswith("__syncwarp()") for nxt in conditional)
