@@ -11,6 +11,7 @@ import ctypes
 import functools
 import math
 import os
+import threading
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -129,6 +130,13 @@ _workspaces = {}
 _retired_workspaces = []
 NUM_SMS = 148
 
+SPLIT_HEADER_BYTES = 65536  # counters at the head of every scratch buffer (CHITU_SPLITKV_HEADER_BYTES)
+# what the largest cut needs on NUM_SMS SMs: a bundle per SM, each with two fragments of two 128-row tiles
+CUT_SCRATCH_BYTES = SPLIT_HEADER_BYTES + NUM_SMS * 4 * 128 * (128 + 1) * 4
+CUT_SCRATCH_STREAMS = 8
+_cut_scratches = {}
+_scratch_lock = threading.Lock()
+
 
 def auto_key_splits(B: int, Sq: int, Sk: int, H: int) -> int:
     """How many key ranges to run as separate CTAs.  A CTA serves 256 query rows of one head; the grid runs in
@@ -181,6 +189,27 @@ def splitkv_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
             _retired_workspaces.append(ws)
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)  # the counters at its head start at zero
         _workspaces[key] = ws
+    return ws
+
+
+def _cut_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
+    """Scratch for the cut query blocks of eager calls on the current stream of ``device``.
+
+    Never the buffer of :func:`splitkv_workspace`, whose address a captured graph may hold: a replay runs on any stream,
+    beside eager calls of this one.  A cut's need has a bound, so the buffer is made once at that size (39 MB).  The
+    buffers made last are kept; an older one goes back to torch's allocator, which reuses it in its stream's order.
+    """
+    key = (_device_key(device), _stream_ptr(device))
+    ws = _cut_scratches.get(key)
+    if ws is None or ws.numel() < nbytes:
+        with _on(device):
+            ws = torch.empty(max(nbytes, CUT_SCRATCH_BYTES), dtype=torch.uint8, device=device)
+            ws[:SPLIT_HEADER_BYTES].zero_()
+        with _scratch_lock:
+            _cut_scratches.pop(key, None)
+            _cut_scratches[key] = ws
+            while len(_cut_scratches) > CUT_SCRATCH_STREAMS:
+                _cut_scratches.pop(next(iter(_cut_scratches)))
     return ws
 
 
@@ -282,12 +311,12 @@ def attn_fwd(
             )
         else:
             # the query blocks of a partly filled last wave are cut along the keys; a graph being captured
-            # keeps them whole (the scratch belongs to eager calls of this stream, which may run beside a replay)
+            # keeps them whole (their scratch belongs to eager calls of this stream, which may run beside a replay)
             ws_ptr, ws_bytes = None, 0
             if automatic and not torch.cuda.is_current_stream_capturing():
                 need = _balanced_workspace_bytes(q.device.index, B, Sq, Sk, H)
                 if need:
-                    ws = splitkv_workspace(q.device, need) if workspace is None else workspace
+                    ws = _cut_scratch(q.device, need) if workspace is None else workspace
                     if ws.numel() * ws.element_size() >= need and ws.device == q.device:
                         ws_ptr, ws_bytes = ws.data_ptr(), ws.numel() * ws.element_size()
             rc = lib.chitu_b200_attn_fwd_balanced(

@@ -1,0 +1,61 @@
+"""Which scratch an attention call gets: host-side rules, with CPU buffers in the place of device memory."""
+
+import types
+
+import pytest
+import torch
+
+
+class Cuda:
+    """The current stream and its capture state, as the code under test sees them."""
+
+    stream = 11
+    capturing = False
+
+
+@pytest.fixture
+def cuda(monkeypatch):
+    from chitudiffusion_b200 import ops
+
+    state = Cuda()
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: types.SimpleNamespace(cuda_stream=state.stream))
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
+    monkeypatch.setattr(ops, "_stream_ptr", lambda dev: state.stream)
+    monkeypatch.setattr(ops, "_workspaces", {})
+    monkeypatch.setattr(ops, "_retired_workspaces", [])
+    monkeypatch.setattr(ops, "_cut_scratches", {})
+    return state
+
+
+CPU = torch.device("cpu")
+
+
+def _header_is_zero(ws):
+    return int(ws[:65536].max()) == 0
+
+
+def test_a_cut_never_uses_the_key_split_buffer(cuda):
+    """The key-split buffer of a stream may be part of a captured graph that is replayed beside eager calls."""
+    from chitudiffusion_b200 import ops
+
+    split = ops.splitkv_workspace(CPU, 50 << 20)  # larger than any cut needs
+    cut = ops._cut_scratch(CPU, 1 << 20)
+    assert cut.data_ptr() != split.data_ptr()
+    assert _header_is_zero(cut)
+    assert ops._cut_scratch(CPU, 30 << 20) is cut  # made once, at the size of the largest cut
+    assert not ops._retired_workspaces
+
+
+def test_the_cut_pool_is_bounded(cuda):
+    from chitudiffusion_b200 import ops
+
+    seen = {}
+    for stream in range(3 * ops.CUT_SCRATCH_STREAMS):
+        cuda.stream = stream
+        seen[stream] = ops._cut_scratch(CPU, 1 << 20)
+    assert len(ops._cut_scratches) == ops.CUT_SCRATCH_STREAMS
+    assert len({t.data_ptr() for t in ops._cut_scratches.values()}) == ops.CUT_SCRATCH_STREAMS
+    assert ops._cut_scratch(CPU, 1 << 20) is seen[stream]
+    # 148 bundles, two fragments of two 128-row tiles each
+    assert ops.CUT_SCRATCH_BYTES == 65536 + 148 * 2 * 2 * 128 * 129 * 4
