@@ -174,11 +174,11 @@ def splitkv_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     """Scratch for key-split partials, one buffer per (device, stream), grown on demand, zero-filled when
     created (the library keeps per-query-block counters in its first 64 KiB and leaves them zero after each call).
 
-    A buffer that has been handed out may be baked into a captured CUDA graph, so a superseded buffer
-    is never freed: it is parked for the life of the process and the larger replacement serves later
-    calls.  Streams do not share a buffer (two streams of one GPU may run key-split calls at once).
-    Objects that own long-lived graphs (the peer exchanges) allocate their own scratch instead and pass
-    it as ``workspace=``.
+    A buffer that has been handed out may have been passed to a captured call as ``workspace=``, so a superseded
+    buffer is never freed: it is parked for the life of the process and the larger replacement serves later
+    calls.  Streams do not share a buffer (two streams of one GPU may run key-split calls at once).  Calls of this
+    module that are captured do not use it (see :func:`_split_scratch`), and objects that own long-lived graphs (the
+    peer exchanges) allocate their own scratch and pass it as ``workspace=``.
     """
     dev = torch.device(device)
     key = (dev.index if dev.index is not None else torch.cuda.current_device(),
@@ -192,12 +192,27 @@ def splitkv_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws
 
 
+def _split_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
+    """Key-split scratch of one call on the current stream of ``device``.
+
+    A call that is being captured gets its own, from the graph's memory and with its counters cleared by the graph
+    itself: a replay runs on any stream, beside eager calls of this one, and memory that is first zeroed by a replay
+    is not zero for an eager call before it.
+    """
+    with _on(device):
+        if not torch.cuda.is_current_stream_capturing():
+            return splitkv_workspace(device, nbytes)
+        ws = torch.empty(max(nbytes, SPLIT_HEADER_BYTES), dtype=torch.uint8, device=device)
+        ws[:SPLIT_HEADER_BYTES].zero_()
+        return ws
+
+
 def _cut_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
     """Scratch for the cut query blocks of eager calls on the current stream of ``device``.
 
-    Never the buffer of :func:`splitkv_workspace`, whose address a captured graph may hold: a replay runs on any stream,
-    beside eager calls of this one.  A cut's need has a bound, so the buffer is made once at that size (39 MB).  The
-    buffers made last are kept; an older one goes back to torch's allocator, which reuses it in its stream's order.
+    Never the buffer of :func:`splitkv_workspace`, whose address a caller's captured graph may hold.  A cut's need has a
+    bound, so the buffer is made once at that size (39 MB).  The buffers made last are kept; an older one goes back to
+    torch's allocator, which reuses it in its stream's order.
     """
     key = (_device_key(device), _stream_ptr(device))
     ws = _cut_scratches.get(key)
@@ -286,7 +301,7 @@ def attn_fwd(
         ws_ptr, ws_bytes = None, 0
         if n_splits > 1:
             need = int(lib.chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, n_splits))
-            ws = workspace if workspace is not None else splitkv_workspace(q.device, need)
+            ws = workspace if workspace is not None else _split_scratch(q.device, need)
             ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()
         with _on(q.device):
             rc = lib.chitu_b200_attn_fwd_qpre(
@@ -300,7 +315,7 @@ def attn_fwd(
     with _on(q.device):
         if n_splits > 1:
             need = int(lib.chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, n_splits))
-            ws = workspace if workspace is not None else splitkv_workspace(q.device, need)
+            ws = workspace if workspace is not None else _split_scratch(q.device, need)
             if ws.numel() * ws.element_size() < need or ws.device != q.device:
                 raise ValueError(f"attn_fwd: workspace must hold {need} bytes on {q.device}")
             rc = lib.chitu_b200_attn_fwd_splitkv(
@@ -710,7 +725,7 @@ def attn_fwd_scatter(
     ws_ptr, ws_bytes = None, 0
     if n_splits > 1:
         need = int(lib.chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, n_splits))
-        ws = workspace if workspace is not None else splitkv_workspace(q.device, need)
+        ws = workspace if workspace is not None else _split_scratch(q.device, need)
         if ws.numel() * ws.element_size() < need or ws.device != q.device:
             raise ValueError(f"attn_fwd_scatter: workspace must hold {need} bytes on {q.device}")
         ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()
@@ -772,7 +787,7 @@ def attn_fwd_exchange(
     ws_ptr, ws_bytes = None, 0
     if n_splits > 1:
         need = int(lib.chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, n_splits))
-        ws = workspace if workspace is not None else splitkv_workspace(q.device, need)
+        ws = workspace if workspace is not None else _split_scratch(q.device, need)
         if ws.numel() * ws.element_size() < need or ws.device != q.device:
             raise ValueError(f"attn_fwd_exchange: workspace must hold {need} bytes on {q.device}")
         ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()

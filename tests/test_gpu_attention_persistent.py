@@ -97,3 +97,33 @@ def test_a_captured_call_keeps_its_query_blocks_whole():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, whole)
+
+
+def test_a_replayed_key_split_call_beside_eager_cut_calls():
+    """A graph captured on one stream, replayed on another beside eager calls of the first: no scratch in common, and
+    none of it is first zeroed by the replay."""
+    from chitudiffusion_b200 import ops
+
+    q, k, v = (t.cuda() for t in _inputs(1, 300, 1500, 5, torch.bfloat16, 6))
+    big = [t.cuda() for t in _inputs(1, 1100, 1500, 37, torch.bfloat16, 7)]
+    want, _ = ops.attn_fwd(q, k, v, n_splits=3)
+    want_big, _ = ops.attn_fwd(*big)
+    torch.cuda.synchronize()
+    one, other = torch.cuda.Stream(), torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=one):  # the stream's first key-split call is a captured one
+        out, _ = ops.attn_fwd(q, k, v, n_splits=3)
+    with torch.cuda.stream(one):
+        early, _ = ops.attn_fwd(q, k, v, n_splits=3)
+    torch.cuda.synchronize()
+    assert torch.equal(early, want)
+    for _ in range(4):
+        with torch.cuda.stream(one):
+            eager = [ops.attn_fwd(*big)[0] for _ in range(4)]
+        with torch.cuda.stream(other):
+            for _ in range(8):
+                graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        assert all(torch.equal(e, want_big) for e in eager)
+    ops.check_status()

@@ -59,3 +59,21 @@ def test_the_cut_pool_is_bounded(cuda):
     assert ops._cut_scratch(CPU, 1 << 20) is seen[stream]
     # 148 bundles, two fragments of two 128-row tiles each
     assert ops.CUT_SCRATCH_BYTES == 65536 + 148 * 2 * 2 * 128 * 129 * 4
+
+
+def test_a_captured_split_call_has_scratch_of_its_own(cuda):
+    from chitudiffusion_b200 import ops
+
+    eager = ops._split_scratch(CPU, 2 << 20)
+    assert ops._split_scratch(CPU, 2 << 20) is eager  # eager calls of a stream share one buffer
+    cuda.capturing = True
+    first, second = ops._split_scratch(CPU, 2 << 20), ops._split_scratch(CPU, 3 << 20)
+    assert len({t.data_ptr() for t in (eager, first, second)}) == 3
+    assert _header_is_zero(first) and first.numel() >= 2 << 20
+    # what a capture zeroes is not zero before the first replay: nothing of it reaches an eager call
+    cuda.capturing = False
+    cuda.stream = 12
+    before = dict(ops._workspaces)
+    cuda.capturing = True
+    ops._split_scratch(CPU, 2 << 20)
+    assert ops._workspaces == before and not ops._cut_scratches
