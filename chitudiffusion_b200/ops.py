@@ -30,6 +30,11 @@ _STATUS_NAMES = {
 
 _status_words = {}
 
+_workspaces = {}
+_retired_workspaces = []
+_cut_scratches = {}
+_scratch_lock = threading.Lock()
+
 # kernels of this library launched so far by this process (the bench reports the count of a timed region)
 launch_count = 0
 
@@ -89,16 +94,25 @@ def status_word(device: torch.device) -> torch.Tensor:
 
 
 def _take_status(key: int) -> None:
-    """Raise (and clear the word) if it is set."""
+    """Raise (and clear the word) if it is set.  A call that gave up may have left counters in its scratch that no later
+    call completes, so the device's buffers are not used again."""
     entry = _status_words.get(key)
     if entry is not None and entry[1].value != 0:
         code = entry[1].value
         entry[1].value = 0
+        with _scratch_lock:
+            for used in [k for k in _workspaces if k[0] == key]:
+                _retired_workspaces.append(_workspaces.pop(used))
+            for used in [k for k in _cut_scratches if k[0] == key]:
+                del _cut_scratches[used]
         raise _lib.ChituB200Error(f"device status {code}: {_STATUS_NAMES.get(code, 'unknown')}")
 
 
 def check_status(device: Optional[torch.device] = None) -> None:
-    """Synchronise and raise if any kernel on `device` reported a timed-out wait."""
+    """Synchronise and raise if any kernel on `device` reported a timed-out wait.
+
+    The scratch buffers that this module keeps for the device are then replaced.  A buffer that the caller passed as
+    ``workspace=`` is the caller's to clear: zero its first ``SPLIT_HEADER_BYTES`` before it is used again."""
     key = torch.cuda.current_device() if device is None else _device_key(device)
     torch.cuda.synchronize(key)
     _take_status(key)
@@ -126,16 +140,12 @@ def set_flag_wait_cycles(cycles: int) -> int:
     return int(_lib.load().chitu_b200_set_flag_wait_cycles(int(cycles)))
 
 
-_workspaces = {}
-_retired_workspaces = []
 NUM_SMS = 148
 
 SPLIT_HEADER_BYTES = 65536  # counters at the head of every scratch buffer (CHITU_SPLITKV_HEADER_BYTES)
 # what the largest cut needs on NUM_SMS SMs: a bundle per SM, each with two fragments of two 128-row tiles
 CUT_SCRATCH_BYTES = SPLIT_HEADER_BYTES + NUM_SMS * 4 * 128 * (128 + 1) * 4
 CUT_SCRATCH_STREAMS = 8
-_cut_scratches = {}
-_scratch_lock = threading.Lock()
 
 
 def auto_key_splits(B: int, Sq: int, Sk: int, H: int) -> int:
@@ -188,7 +198,8 @@ def splitkv_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
         if ws is not None:
             _retired_workspaces.append(ws)
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=dev)  # the counters at its head start at zero
-        _workspaces[key] = ws
+        with _scratch_lock:
+            _workspaces[key] = ws
     return ws
 
 
@@ -212,7 +223,8 @@ def _cut_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
 
     Never the buffer of :func:`splitkv_workspace`, whose address a caller's captured graph may hold.  A cut's need has a
     bound, so the buffer is made once at that size (39 MB).  The buffers made last are kept; an older one goes back to
-    torch's allocator, which reuses it in its stream's order.
+    torch's allocator, which reuses it in its stream's order.  None is kept past a wait that ran out (see
+    :func:`check_status`).
     """
     key = (_device_key(device), _stream_ptr(device))
     ws = _cut_scratches.get(key)

@@ -77,3 +77,29 @@ def test_a_captured_split_call_has_scratch_of_its_own(cuda):
     cuda.capturing = True
     ops._split_scratch(CPU, 2 << 20)
     assert ops._workspaces == before and not ops._cut_scratches
+
+
+def test_a_reported_timeout_takes_the_scratch_out_of_use(cuda, monkeypatch):
+    """The call that gave up may have left counters behind; the next one must not find them."""
+    import ctypes
+
+    from chitudiffusion_b200 import _lib, ops
+
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda dev=None: None)
+    word = ctypes.c_int32(0)
+    monkeypatch.setattr(ops, "_status_words", {0: (None, word), 1: (None, ctypes.c_int32(0))})
+    split, cut = ops.splitkv_workspace(CPU, 1 << 20), ops._cut_scratch(CPU, 1 << 20)
+    ops._cut_scratches[(1, 5)] = other = torch.empty(8, dtype=torch.uint8)
+    ops.poll_status(torch.device("cuda", 0))  # nothing reported: the buffers stay
+    assert ops._cut_scratch(CPU, 1 << 20) is cut and ops.splitkv_workspace(CPU, 1 << 20) is split
+    for raising in (ops.poll_status, ops.check_status):
+        for ws in (split, cut):
+            ws[:4].fill_(1)
+        word.value = 3
+        with pytest.raises(_lib.ChituB200Error, match="softmax"):
+            raising(torch.device("cuda", 0))
+        assert word.value == 0
+        fresh_split, fresh_cut = ops.splitkv_workspace(CPU, 1 << 20), ops._cut_scratch(CPU, 1 << 20)
+        assert _header_is_zero(fresh_split) and _header_is_zero(fresh_cut)
+        split, cut = fresh_split, fresh_cut
+    assert ops._cut_scratches[(1, 5)] is other  # another device's buffers are not touched
