@@ -44,10 +44,18 @@ def _launched(n: int = 1) -> None:
     launch_count += n
 
 
-def _stream_ptr(device: torch.device) -> int:
+def _device_key(device) -> int:
+    """Index of a device given in any of the forms torch takes: an object, a name, an index, None for the current one."""
+    if not isinstance(device, torch.device):
+        device = torch.device("cuda" if device is None else device)
+    if device.type != "cuda":
+        raise ValueError(f"Expected a cuda device, but got: {device}")
+    return torch.cuda.current_device() if device.index is None else device.index
+
+
+def _stream_ptr(device) -> int:
     # the handle alone: building a torch Stream object costs ten times as much and every call needs it
-    index = device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    return torch._C._cuda_getCurrentRawStream(_device_key(device))
 
 
 class _NoGuard:
@@ -61,10 +69,11 @@ class _NoGuard:
 _NO_GUARD = _NoGuard()
 
 
-def _on(device: torch.device):
+def _on(device):
     """``torch.cuda.device(device)`` where that changes anything (entering and leaving it costs some microseconds)."""
-    if device.index is None or torch._C._cuda_getDevice() == device.index:
-        return _NO_GUARD
+    if isinstance(device, torch.device) and device.type == "cuda":
+        if device.index is None or torch._C._cuda_getDevice() == device.index:
+            return _NO_GUARD
     return torch.cuda.device(device)
 
 
@@ -72,11 +81,6 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
     for t in tensors:
         if t is not None and not t.is_cuda:
             raise RuntimeError("chitudiffusion_b200 runs on CUDA tensors only (there is no CPU path)")
-
-
-def _device_key(device) -> int:
-    index = torch.device(device).index if not isinstance(device, torch.device) else device.index
-    return torch.cuda.current_device() if index is None else index
 
 
 def status_word(device: torch.device) -> torch.Tensor:

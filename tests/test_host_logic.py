@@ -64,3 +64,28 @@ def test_cached_ring_refuses_bad_plans():
         ring(None, None, None, plan=[False, True, True, True])  # the local block is always computed
     with pytest.raises(RuntimeError):
         ring(None, None, None, plan=[True, False, True, True])  # nothing kept yet for offset 1
+
+
+def test_devices_in_every_form_that_torch_takes(monkeypatch):
+    """The entry points that are given a device (barriers, copies, waits) rather than a tensor take an index or a name too."""
+    import torch
+
+    from chitudiffusion_b200 import ops
+
+    entered = []
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: entered.append(d) or ops._NO_GUARD)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 1000 + index, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 3, raising=False)
+    for device, index in ((torch.device("cuda", 1), 1), (torch.device("cuda"), 3), ("cuda:2", 2), ("cuda", 3), (0, 0), (None, 3)):
+        assert ops._device_key(device) == index and ops._stream_ptr(device) == 1000 + index
+        with ops._on(device):
+            pass
+    # a guard is entered for another device than the current one, and for the forms that only torch itself resolves
+    assert entered == [torch.device("cuda", 1), "cuda:2", "cuda", 0, None]
+    with ops._on(torch.device("cuda", 3)):
+        assert len(entered) == 5
+    ops._on(torch.device("cpu"))  # left to torch, which refuses it
+    assert entered[-1] == torch.device("cpu")
+    with pytest.raises(ValueError, match="cuda device"):
+        ops._stream_ptr(torch.device("cpu"))

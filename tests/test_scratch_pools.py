@@ -22,6 +22,8 @@ def cuda(monkeypatch):
     monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: types.SimpleNamespace(cuda_stream=state.stream))
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state.capturing)
     monkeypatch.setattr(ops, "_stream_ptr", lambda dev: state.stream)
+    monkeypatch.setattr(ops, "_device_key", lambda dev: dev.index or 0)
+    monkeypatch.setattr(ops, "_on", lambda dev: ops._NO_GUARD)
     monkeypatch.setattr(ops, "_workspaces", {})
     monkeypatch.setattr(ops, "_retired_workspaces", [])
     monkeypatch.setattr(ops, "_cut_scratches", {})
