@@ -278,7 +278,10 @@ _I64x4 = ctypes.c_int64 * 4
 
 def i64_array(values: Sequence[int]):
     if len(values) == 4:
-        return _I64x4(*values)
+        try:
+            return _I64x4(*values)
+        except TypeError:  # strides that are whole numbers but no Python ints
+            pass
     return (ctypes.c_int64 * len(values))(*[int(v) for v in values])
 
 

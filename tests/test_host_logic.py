@@ -89,3 +89,16 @@ def test_devices_in_every_form_that_torch_takes(monkeypatch):
     assert entered[-1] == torch.device("cpu")
     with pytest.raises(ValueError, match="cuda device"):
         ops._stream_ptr(torch.device("cpu"))
+
+
+def test_strides_may_be_any_whole_numbers():
+    import numpy as np
+    import torch
+
+    from chitudiffusion_b200 import _lib
+
+    want = [640, 128, 0, -8]
+    for values in (want, tuple(want), np.array(want), [float(v) for v in want], list(torch.tensor(want)),
+                   torch.empty(2, 3, 4, 5).stride()):
+        assert list(_lib.i64_array(values)) == [int(v) for v in values]
+    assert list(_lib.i64_array(np.array([1, 2, 3]))) == [1, 2, 3]
