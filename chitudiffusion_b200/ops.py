@@ -244,6 +244,13 @@ def _cut_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws
 
 
+def _holds(ws: torch.Tensor, nbytes: int, device: torch.device) -> bool:
+    """Whether a caller's buffer will do as scratch of a call that can also run without (a call on one key range has
+    always taken any ``workspace``, and left it alone)."""
+    return (ws.device == device and ws.numel() * ws.element_size() >= nbytes and ws.data_ptr() % 16 == 0
+            and ws.is_contiguous())
+
+
 def splitkv_workspace_bytes(B: int, Sq: int, H: int, D: int, n_splits: int) -> int:
     """Bytes of scratch a key-split call of this shape needs (0 for one split)."""
     return int(_lib.load().chitu_b200_attn_splitkv_workspace_bytes(B, Sq, H, D, int(n_splits)))
@@ -269,7 +276,8 @@ def attn_fwd(
     """``softmax(scale * q k^T) v`` for ``[B,S,H,128]`` bf16/fp16 tensors of any (16-byte aligned) strides.
 
     Returns ``(out [B,Sq,H,D] contiguous, lse [B,H,Sq] fp32 | None)``.  ``workspace`` is an optional
-    caller-owned uint8 scratch for the key-split partials (see :func:`splitkv_workspace`); its first 64 KiB
+    caller-owned uint8 scratch for the key-split partials (see :func:`splitkv_workspace`) and for the cut query blocks of
+    a call on one key range, which is not cut where the buffer will not do; its first 64 KiB
     hold counters that must be zero before the first use (``torch.zeros``) and are left zero by every call.  With ``q_pre``
     (keys ``norm_mode, rope_mode, weight, rstd, eps, rope_table, grid, axis_split, pos_offset, round_mid``)
     ``q`` is the raw projection and its pre-attention transform runs inside the kernel
@@ -348,7 +356,7 @@ def attn_fwd(
                 need = _balanced_workspace_bytes(q.device.index, B, Sq, Sk, H)
                 if need:
                     ws = _cut_scratch(q.device, need) if workspace is None else workspace
-                    if ws.numel() * ws.element_size() >= need and ws.device == q.device:
+                    if _holds(ws, need, q.device):
                         ws_ptr, ws_bytes = ws.data_ptr(), ws.numel() * ws.element_size()
             rc = lib.chitu_b200_attn_fwd_balanced(
                 q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),

@@ -127,3 +127,15 @@ def test_a_replayed_key_split_call_beside_eager_cut_calls():
         assert torch.equal(out, want)
         assert all(torch.equal(e, want_big) for e in eager)
     ops.check_status()
+
+
+def test_any_workspace_is_taken_by_a_call_on_one_key_range():
+    from chitudiffusion_b200 import ops
+
+    q, k, v = (t.cuda() for t in _inputs(1, 1100, 1500, 37, torch.bfloat16, 8))
+    whole, _ = ops.attn_fwd(q, k, v, n_splits=1)
+    big = torch.zeros(2 * _need(1, 1100, 1500, 37) + 16, dtype=torch.uint8, device="cuda")
+    for ws in (big[8:], big[:16], big.view(-1, 2)[:, 0], torch.zeros(0, dtype=torch.uint8, device="cuda")):
+        out, _ = ops.attn_fwd(q, k, v, workspace=ws)
+        assert torch.equal(out, whole)
+    assert int(big.max().item()) == 0

@@ -105,3 +105,16 @@ def test_a_reported_timeout_takes_the_scratch_out_of_use(cuda, monkeypatch):
         assert _header_is_zero(fresh_split) and _header_is_zero(fresh_cut)
         split, cut = fresh_split, fresh_cut
     assert ops._cut_scratches[(1, 5)] is other  # another device's buffers are not touched
+
+
+def test_a_callers_buffer_that_will_not_do_is_left_alone():
+    """Too small, off its alignment or with gaps: the call runs its query blocks whole instead of being refused."""
+    from chitudiffusion_b200 import ops
+
+    raw = torch.zeros(4096 + 64, dtype=torch.uint8)
+    base = raw[(-raw.data_ptr()) % 16:][:4096]
+    assert ops._holds(base, 4096, CPU)
+    assert not ops._holds(base, 4097, CPU)
+    assert not ops._holds(raw[(-raw.data_ptr()) % 16 + 8:], 1024, CPU)
+    assert not ops._holds(base.view(64, 64)[:, :32], 1024, CPU)
+    assert not ops._holds(base, 1024, torch.device("cuda", 0))
