@@ -99,7 +99,10 @@ class B200AttnBackend:
         """Pre-attention transform and attention of one layer; same contract as
         ``B200ContextParallel.attention_from_projections`` (so model code calls one name on one or many GPUs).
 
-        Two placements of q's transform exist and give bit-identical results.  Default: q and k both go
+        Two placements of q's transform exist.  The transformed q is the same bit for bit, and so is the result where
+        both forms run the same attention kernel (grids of up to one query block per SM); on larger grids the
+        pre-pass form takes the persistent kernel, and the results agree to the 16-bit rounding of probabilities
+        and outputs (2^-7 of the largest value).  Default: q and k both go
         through the pre-pass kernel (one launch).  With ``CHITU_B200_Q_PRELOAD=fused`` (or
         ``self.q_in_kernel = True``) a layer that arrives in ONE piece has its query transform done INSIDE the
         attention kernel: only k goes through the pre-pass, q is read once - raw - by the attention

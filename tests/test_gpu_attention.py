@@ -344,3 +344,29 @@ def test_query_transform_inside_the_kernel_equals_the_pre_pass(backend):
                                                  **wan.batch_args(S, grid))
     assert torch.equal(default, plain)
     ops.check_status(dev)
+
+
+@pytest.mark.parametrize("S,H", [(1800, 24), (1100, 40)])  # whole query blocks / the last wave's cut
+def test_query_transform_inside_the_kernel_on_more_than_one_wave(backend, S, H):
+    """There the pre-pass form runs the persistent kernel: the same operands in another schedule.  Probabilities (half a
+    bf16 ulp each, summed over the keys with a common scale) and the result (half an ulp) are rounded anew: 2^-8 of the
+    largest value between the two and room for one more rounding."""
+    from chitudiffusion_b200 import ops, pre_attention
+
+    D = 128
+    C = H * D
+    gen = torch.Generator().manual_seed(S)
+    qkv = _rand((1, S, 3 * C), torch.bfloat16, gen, 0.7).cuda()
+    ids = torch.stack([torch.zeros(S, dtype=torch.long), torch.arange(S) // 45, torch.arange(S) % 45], 1)
+    pre = pre_attention.JointPreAttention(H, D, pre_attention.axis_rope_table(ids, (16, 56, 56)).cuda())
+    wq, wk = ((1.0 + 0.1 * torch.randn(D, generator=gen)).cuda() for _ in range(2))
+    parts = qkv[..., :C], qkv[..., C:2 * C], qkv[..., 2 * C:]
+    results = []
+    for backend.q_in_kernel in (True, False):
+        results.append(backend.attention_from_projections(pre.jobs(*parts[:2], wq, wk), parts[2], **pre.batch_args()))
+    q, k, v = pre(*parts, wq, wk)
+    ref = oracle.sdpa_fp32(q.cpu(), k.cpu(), v.cpu())
+    for out in results:
+        _check(out, ref)
+    assert (results[0].float() - results[1].float()).abs().max().item() <= 2 ** -7 * ref.abs().max().item()
+    ops.check_status()
