@@ -27,13 +27,13 @@ def test_peer_barrier_gives_up_and_reports():
         with pytest.raises(_lib.ChituB200Error, match="flag wait"):
             ops.check_status(dev)
         ops.check_status(dev)  # the word was cleared by the raise
-        # the deferred form used on the product path: the poll after the failing launch enqueues a copy of
-        # the word, a later poll sees it
+        # the form used on the product path looks at the word as it is, without synchronising: the first poll
+        # after the report raises, the next finds the word cleared
         ops.peer_barrier([f.data_ptr() for f in flags], rank=0, world=2, device=dev)
-        ops.poll_status(dev)
         torch.cuda.synchronize()
         with pytest.raises(_lib.ChituB200Error, match="flag wait"):
             ops.poll_status(dev)
+        ops.poll_status(dev)
         torch.cuda.synchronize()
         ops.check_status(dev)
         # a barrier that IS answered (one rank) still passes and the device still computes
