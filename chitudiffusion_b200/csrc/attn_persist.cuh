@@ -8,10 +8,11 @@
 // out one query block, the next one's Q, K and V are on their way and its first scores are being computed.
 //
 // Work units.  Unit u of the grid is a run of key-tile steps in the flattened order (query block, key tile):
-//   u < n_bundles   steps [u * bundle_steps, (u + 1) * bundle_steps) of the first cut_items query blocks,
-//   otherwise       one whole query block.
-// Query blocks that do not fill the last wave of the machine are cut into equal bundles, one per SM, so that
-// all SMs finish together; a bundle touches at most two query blocks and leaves a fragment of each in scratch
+//   u < n_whole   one whole query block,
+//   otherwise     with b = u - n_whole, steps [b * bundle_steps, (b + 1) * bundle_steps) of the first cut_items query blocks.
+// Query blocks that do not fill the last wave of the machine are cut into equal bundles, at most one per SM, so that
+// all SMs finish together.  The bundles come last: a CTA asks for its next unit while it works on one, so whole blocks
+// behind bundles would go to CTAs that have a whole block in hand as often as to those that took a bundle.  A bundle touches at most two query blocks and leaves a fragment of each in scratch
 // memory, and the warp that completes the last fragment of its 32 rows merges them (nobody waits).
 //
 // Units are handed out by the hardware: the grid has one CTA per unit, and a running CTA takes over units that
@@ -67,9 +68,10 @@ struct AttnPersistParams {
   int n_kv;          // key tiles
   int n_qblocks;     // query blocks per head; item = (head * B + batch) * n_qblocks + block, so that CTAs which run
                      // together share heads' keys in L2
-  int cut_items;     // the first cut_items query blocks are cut into
-  int n_bundles;     // bundles of
-  int bundle_steps;  // key-tile steps each (<= n_kv)
+  int n_whole;       // units that are whole query blocks; the others are the
+  int n_bundles;     // bundles into which the first cut_items query blocks are cut, of
+  int bundle_steps;  // key-tile steps each (< n_kv)
+  int cut_items;
   FastDiv by_n_kv, by_n_qblocks, by_batch, by_bundle_steps;
   // scratch (cut_items > 0): counters [cut_items][2 tiles][4 warps], zero between calls; a fragment's normalised fp32 rows
   // [bundle * 2 + k][2 tiles][32 chunks][128 rows] float4 (k = 0, 1: the bundle's first / second query block) and
@@ -222,12 +224,12 @@ __device__ __forceinline__ void persist_softmax_step(const TileRefs& r, int step
 struct UnitWalk {
   int pos, end;
   __device__ __forceinline__ UnitWalk(const AttnPersistParams& p, int unit) {
-    if (unit < p.n_bundles) {
-      pos = unit * p.bundle_steps;
-      end = min(pos + p.bundle_steps, p.cut_items * p.n_kv);
-    } else {
-      pos = (p.cut_items + unit - p.n_bundles) * p.n_kv;
+    if (unit < p.n_whole) {
+      pos = (p.cut_items + unit) * p.n_kv;
       end = pos + p.n_kv;
+    } else {
+      pos = (unit - p.n_whole) * p.bundle_steps;
+      end = min(pos + p.bundle_steps, p.cut_items * p.n_kv);
     }
   }
   __device__ __forceinline__ bool next(const AttnPersistParams& p, int& item, int& kv0, int& n) {

@@ -216,19 +216,23 @@ int64_t splitkv_workspace_bytes(int B, int Sq, int H, int D, int n_splits) {
 // (see AttnPersistParams).
 //
 // The blocks that do not fill the last wave of SMs - one CTA each - are cut into one bundle of key-tile steps per
-// SM, none shorter than an eighth of the keys (the CTA that completes a query block merges all its fragments).
-// A cut costs about kCutSteps steps (two epilogues to scratch memory instead of one to the output, and the merge).
+// SM, none shorter than an eighth of the keys (the warp that completes a query block's rows merges all their fragments).
+// In steps, a cut costs 3 (two epilogues to scratch memory instead of one to the output), 3/4 per fragment of a block
+// (the merge) and n_kv / 24 (blocks alone in a last wave run their steps that much faster); it is taken where that
+// saves 4 %.  Measured, whole -> cut, us, blocks x tiles: 150 x 12 47 -> 45, x 24 85 -> 68, x 64 209 -> 140;
+// 240 x 24 89 -> 88; 340 x 36 183 -> 168; 600 x 64 553 -> 487; not taken: 168 x 9 39 -> 46, 240 x 16 64 -> 67, 400 x 24
+// 130 -> 134, 432 x 36 202 -> 213.  (Of 168 pairs of 150 to 744 blocks and 2 to 128 tiles the rule takes two that
+// lose, 168 x 12 and x 16, by 2 %.)
 // Grids that do not fill the machine once are the business of the key-split entry points.
 //
 // The persistent kernel takes every grid that fills the machine at least once; below that a CTA has a single query
 // block and attn_fwd_kernel (whose key ranges such grids are offered) does the same work.  Measured, attn_fwd_kernel ->
 // persistent, us: 512 keys 147 -> 103 (S = 32760, H = 12); 36 key tiles 209 -> 195 (S = 4608, H = 24, 2.9 waves);
-// 61 tiles 322 -> 306, cut PERSIST_CUT (2.5 waves); 256 tiles 4850 -> 4665 (10.4 waves).
+// 61 tiles 322 -> 303, cut 289 (2.5 waves); 256 tiles 4850 -> 4665 (10.4 waves).
 struct CutPlan {
   bool persistent = false;
   int cut_items = 0, n_bundles = 0, bundle_steps = 1;
 };
-constexpr int kCutSteps = 5;
 CutPlan plan_cut(long long items, int n_kv, int sms, bool may_cut) {
   CutPlan c;
   if (sms <= 0) return c;
@@ -237,8 +241,10 @@ CutPlan plan_cut(long long items, int n_kv, int sms, bool may_cut) {
   if (waves == 0 || rem == 0 || !may_cut) return c;
   const long long per_sm = (rem * n_kv + sms - 1) / sms, floor_steps = (n_kv + 7) / 8;
   const long long steps = per_sm > floor_steps ? per_sm : floor_steps;
-  const long long whole = (waves + 1) * n_kv, cut = waves * n_kv + steps + kCutSteps;
-  if (cut * 100 >= whole * 98) return c;
+  const long long fragments = (n_kv + steps - 1) / steps;
+  // in 24ths of a step
+  const long long whole = 24 * (waves + 1) * n_kv, cut = 24 * (waves * n_kv + steps + 3) + 18 * fragments + n_kv;
+  if (steps >= n_kv || cut * 100 >= whole * 96) return c;
   c.cut_items = static_cast<int>(rem);
   c.bundle_steps = static_cast<int>(steps);
   c.n_bundles = static_cast<int>((rem * n_kv + steps - 1) / steps);
@@ -280,6 +286,7 @@ int attn_persist_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
   p.n_qblocks = (Sq + chitu::kQTiles * chitu::kTileM - 1) / (chitu::kQTiles * chitu::kTileM);
   const long long items = query_blocks(B, Sq, H);
   p.cut_items = cut.cut_items;
+  p.n_whole = static_cast<int>(items - cut.cut_items);
   p.n_bundles = cut.n_bundles;
   p.bundle_steps = cut.bundle_steps;
   p.by_n_kv.set(p.n_kv);
@@ -302,7 +309,7 @@ int attn_persist_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUte
       fp16 ? ensure_dynamic_smem(chitu::attn_persist_kernel<true>, chitu::kPersistSmemBytes, attr_done[1], attr_mu)
            : ensure_dynamic_smem(chitu::attn_persist_kernel<false>, chitu::kPersistSmemBytes, attr_done[0], attr_mu);
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "attn_fwd: cudaFuncSetAttribute");
-  const dim3 grid(static_cast<unsigned>(items - cut.cut_items + cut.n_bundles));
+  const dim3 grid(static_cast<unsigned>(p.n_whole + cut.n_bundles));
   if (fp16)
     chitu::attn_persist_kernel<true><<<grid, chitu::kAttnThreads, chitu::kPersistSmemBytes, st>>>(tq, tk, tv, to, p);
   else

@@ -139,3 +139,30 @@ def test_any_workspace_is_taken_by_a_call_on_one_key_range():
         out, _ = ops.attn_fwd(q, k, v, workspace=ws)
         assert torch.equal(out, whole)
     assert int(big.max().item()) == 0
+
+
+# fewer bundles than SMs behind one, two and three waves of whole blocks; one bundle per SM; one-tile query blocks among the cut
+@pytest.mark.parametrize("B,Sq,Sk,H", [(1, 2560, 2100, 15), (1, 2500, 1700, 30), (1, 3840, 1800, 31), (1, 1500, 2500, 37), (2, 300, 2200, 40)])
+def test_bundles_behind_whole_blocks(B, Sq, Sk, H):
+    from chitudiffusion_b200 import ops
+
+    q, k, v = _inputs(B, Sq, Sk, H, torch.bfloat16, Sq)
+    ref, ref_lse = oracle.sdpa_fp32(q, k, v, return_lse=True)
+    need = _need(B, Sq, Sk, H)
+    assert need > 0
+    ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+    ws[65536:] = 0xff  # NaN wherever a fragment is read that was not written
+    for _ in range(2):
+        out, lse = ops.attn_fwd(q.cuda(), k.cuda(), v.cuda(), return_lse=True, workspace=ws)
+        assert (out.float().cpu() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item()
+        assert (lse.cpu() - ref_lse).abs().max().item() <= 1e-3
+    assert int(ws[:65536].max().item()) == 0
+    ops.check_status()
+
+
+def test_a_cut_that_does_not_pay_is_not_taken():
+    """Few key tiles: two epilogues and the merge cost more than the last wave's idle SMs."""
+    assert _need(1, 1664, 1100, 24) == 0  # 168 blocks x 9 tiles: 39 us whole, 46 us cut
+    assert _need(1, 2560, 2048, 24) == 0  # 240 x 16: 64, 67
+    assert _need(1, 4608, 4608, 24) == 0  # 432 x 36: 202, 213
+    assert _need(1, 2560, 8192, 15) > 0  # 150 x 64: 209, 140
