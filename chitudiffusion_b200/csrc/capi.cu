@@ -1131,16 +1131,39 @@ int chitu_b200_layernorm_modulate(const void* x, int x_dtype, void* out, int out
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int per_vec = x_dtype == CHITU_DTYPE_FP32 ? 4 : 8;
   const int64_t batches = rows / rows_per_batch;
-  // the column form wants whole 16-byte vectors, whole batches and a block's worth of columns (narrow rows would leave
-  // most of its threads idle)
   const int n_vec = C / per_vec;
-  if (C % per_vec == 0 && n_vec >= 64 && n_vec <= 2048 && rows % rows_per_batch == 0 && batches <= 65535 &&
-      !(reinterpret_cast<uintptr_t>(out) & 15)) {
+  const bool out16 = !(reinterpret_cast<uintptr_t>(out) & 15);
+  // The column form wants whole 16-byte vectors, whole batches and at least a warp's worth of columns.  A warp per row
+  // (whole groups of 32 vectors, 16 at most) is faster where it fits and (us, warp / column)
+  //   * rows are narrower than 64 vectors and few, so that most of a column block's warps are missing (512 x 128 fp32
+  //     2.6 / 2.7, 4096 rows 4.9 / 3.3),
+  //   * very many batches hold one or two rows, each with modulation vectors of its own that a column block loads for
+  //     a quarter of its row slots (1024 x 1 x 3072 bf16 7.6 / 12.3, 256 x 1 6.6 / 4.1), or
+  //   * fp32 rows of 385 to 512 vectors fill the machine: two blocks of 64 registers a thread, two rows in flight each, are
+  //     all that fits (8192 x 2048 21.4 / 24.5, 2048 rows 8.4 / 8.8, 1024 rows 7.6 / 5.8); not so with more batches
+  //     than SMs, where the warps' modulation vectors come from memory (300 x 64 x 2048 101 / 81).
+  // A block per row takes the rest of the short batches (256 x 1 x 3072 fp32 4.9, column 5.8; 64 x 1 3.6, 3.1) and what
+  // fits neither.
+  const bool column_fits = C % per_vec == 0 && n_vec >= 32 && n_vec <= 2048 && rows % rows_per_batch == 0 && batches <= 65535 && out16;
+  const bool warp_fits = C % (32 * per_vec) == 0 && n_vec <= 32 * chitu::kLnWarpMaxVec && out16;
+  const bool warp_form = warp_fits && (!column_fits || (n_vec < 64 && rows < 2048) || (rows_per_batch <= 2 && batches > 384) ||
+                                       (x_dtype == CHITU_DTYPE_FP32 && n_vec > 384 && rows >= 1500 && (batches <= 148 || rows < 8192)));
+  if (warp_form) {
+    const int grid = static_cast<int>(std::min<int64_t>((rows + 7) / 8, 148 * 8));
+    if (x_dtype == CHITU_DTYPE_BF16)
+      chitu::layernorm_affine_warp_kernel<0><<<grid, 256, 0, st>>>(p);
+    else if (x_dtype == CHITU_DTYPE_FP16)
+      chitu::layernorm_affine_warp_kernel<1><<<grid, 256, 0, st>>>(p);
+    else
+      chitu::layernorm_affine_warp_kernel<2><<<grid, 256, 0, st>>>(p);
+  } else if (column_fits && (warp_fits || rows_per_batch > 1 || batches <= 148)) {
     const int two = n_vec > 1024;
     const int threads = ((two ? (n_vec + 1) / 2 : n_vec) + 31) / 32 * 32;
     const int rows_each = threads <= 384 ? 4 : 2;
     const int64_t groups = (rows_per_batch + rows_each - 1) / rows_each;
-    const int64_t resident = std::max<int64_t>(1, 148 * (threads <= 384 ? (x_dtype == CHITU_DTYPE_FP32 ? 1152 : 768) / threads : 1) / batches);
+    // blocks that an SM holds at once (registers: 80 a thread in the form of up to 384 threads, 56 with fp32 rows, else 64)
+    const int per_sm = threads <= 384 ? (x_dtype == CHITU_DTYPE_FP32 ? 1152 : 768) / threads : threads <= 512 ? 2 : 1;
+    const int64_t resident = std::max<int64_t>(1, 148 * per_sm / batches);
     const dim3 grid(static_cast<unsigned>(std::min<int64_t>(groups, resident)), static_cast<unsigned>(batches));
 #define CHITU_LN(DT) \
     (two              ? chitu::layernorm_affine_rows_kernel<DT, 2, 1024><<<grid, threads, 0, st>>>(p) \

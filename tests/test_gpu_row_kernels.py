@@ -70,3 +70,15 @@ def test_lse_combine_rows(B, S, H, dtype):
     ref = sum(w[i] * outs[i].double() for i in range(3))
     assert (acc.double().cpu() - ref).abs().max().item() <= 2e-6 * ref.abs().max().item() + 1e-6
     assert (acc_lse.double().cpu() - torch.logsumexp(l64, 0)).abs().max().item() <= 1e-5
+
+
+# where the dispatch changes hands: narrow rows, few and many; one and two rows in very many batches (a warp's and a
+# block's worth of columns); fp32 rows of 512 vectors below and above the machine's fill; a last batch that is not whole
+@pytest.mark.parametrize("C,dtype,B,L", [
+    (128, torch.float32, 1, 300), (128, torch.float32, 1, 2048), (256, torch.bfloat16, 3, 700), (1536, torch.float32, 400, 1),
+    (3072, torch.bfloat16, 400, 2), (3072, torch.float32, 160, 1), (5120, torch.bfloat16, 160, 1), (2048, torch.float32, 1, 1499),
+    (2048, torch.float32, 3, 501), (4096, torch.bfloat16, 1, 1600), (512, torch.float32, 520, 3), (1024, torch.bfloat16, 520, 3),
+    (64, torch.float16, 700, 2),
+])
+def test_layernorm_and_gate_where_forms_change(C, dtype, B, L):
+    test_layernorm_and_gate(C, dtype, B, L)
