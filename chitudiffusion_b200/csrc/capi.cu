@@ -1208,13 +1208,23 @@ int chitu_b200_gate_residual(void* x, int x_dtype, const void* y, int y_dtype, i
   p.y_fp16 = y_dtype == CHITU_DTYPE_FP16;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t batches = rows / rows_per_batch;
-  // the column form wants 16-byte vectors of y, whole batches and a row that fits a block
-  if (!(C & 7) && C <= 8192 && rows % rows_per_batch == 0 && batches <= 65535 && !(reinterpret_cast<uintptr_t>(y) & 15)) {
-    const int n_vec = C >> 3;
-    const int rows_par = n_vec >= 512 ? 1 : 512 / n_vec;
+  const bool fp32_x = x_dtype == CHITU_DTYPE_FP32;
+  const int n_vec = C >> 3;
+  const int rows_par = n_vec >= 512 || n_vec == 0 ? 1 : 512 / n_vec;
+  // The column form wants 16-byte vectors of y, whole batches and a row that fits a block.  Many batches that do not give
+  // a block's threads a row each (fp32: one and a half) are left to the general kernel, which deals out elements
+  // and not blocks (us, column / general: 1024 x 1 x 3072 fp32 12.7 / 8.7, 256 x 1 4.2 / 6.0; 4096 x 1 x 1024 bf16 35.4 / 14.9).
+  const bool column = !(C & 7) && C <= 8192 && rows % rows_per_batch == 0 && batches <= 65535 && !(reinterpret_cast<uintptr_t>(y) & 15) &&
+                      !(batches >= 512 && (fp32_x ? rows_per_batch * n_vec <= 768 : rows_per_batch < rows_par));
+  if (column) {
     const int threads = n_vec * rows_par;
     const int64_t groups = (rows_per_batch + rows_par - 1) / rows_par;
-    const int64_t resident = std::max<int64_t>(1, 148 * (2048 / threads) / batches);
+    // An SM holds one block of 512 threads (74 registers each, 86 with an fp32 stream) or two of 384.  More blocks than
+    // two per SM only split the rows until a block's four row slots stay empty (us at four / two per SM: 1024 x 3072 fp32
+    // 10.5 / 8.3, the general kernel 8.4; 1024 x 3072 bf16 6.8 / 5.4; 4096 x 3072 bf16 15.6 / 14.3).  Where every SM has a batch
+    // anyway, blocks even out the last wave as long as their slots stay full
+    // (us at one / two per batch: 200 x 64 x 2048 fp32 50 / 44; 256 x 4 6.6 / 8.5).
+    const int64_t resident = std::max<int64_t>(1, batches <= 148 ? 296 / batches : std::min<int64_t>(148 * (2048 / threads) / batches, groups / 4));
     const dim3 grid(static_cast<unsigned>(std::min<int64_t>(groups, resident)), static_cast<unsigned>(batches));
 #define CHITU_GATE_Y(DT, FP16) \
     (threads <= 512 ? chitu::gate_residual_rows_kernel<DT, FP16, 512><<<grid, threads, 0, st>>>(p, rows_par) \
