@@ -170,9 +170,11 @@ __device__ __forceinline__ float2 exp2_poly2(float2 x) {
 //   bar_p       the tile's two hand-over barriers (keys [0, 64) and [64, 128); every thread arrives)
 //   first       no accumulator yet
 //   valid       keys of this tile that exist (kTileN: all)
+//   m_used      the maximum that is subtracted; neg_m what that adds to a scaled score, carried along because it changes
+//               in few steps and would stand between the maximum and the exponentials in each
 template <bool kFp16>
 __device__ __forceinline__ void softmax_step(uint32_t t_s, uint32_t t_o, uint32_t bar_p, bool first, int valid, float sl2,
-                                             float& m_used, float& l_sum) {
+                                             float& m_used, float& neg_m, float& l_sum) {
   // Row of 128 scores into registers, 32 columns per load; the load of chunk
   // c+1 is in flight while the running maximum of chunk c is taken.
   uint32_t s[4][32];
@@ -195,8 +197,10 @@ __device__ __forceinline__ void softmax_step(uint32_t t_s, uint32_t t_o, uint32_
   }
   const float mx = fmaxf(mx0, mx1);
 
+  // (a row without a finite score so far has nothing to subtract: its probabilities are zero, not NaN)
   if (first) {
     m_used = mx;
+    neg_m = mx == -INFINITY ? 0.f : -mx * sl2;
   } else {
     const bool need = (mx - m_used) * sl2 > kRescaleThreshold;
     if (__any_sync(0xffffffffu, need)) {
@@ -211,14 +215,15 @@ __device__ __forceinline__ void softmax_step(uint32_t t_s, uint32_t t_o, uint32_
         tmem_st32(t_o + c * 32, o);
       }
       l_sum *= f;
-      if (need) m_used = mx;
+      if (need) {
+        m_used = mx;
+        neg_m = -mx * sl2;
+      }
     }
   }
 
   // p = 2^(s*scale - m*scale): packed two-wide FMA / add, one MUFU per element
   const float2 sl2_2 = make_float2(sl2, sl2);
-  // (a row without a finite score so far has nothing to subtract: its probabilities are zero, not NaN)
-  const float neg_m = m_used == -INFINITY ? 0.f : -m_used * sl2;
   const float2 neg_m2 = make_float2(neg_m, neg_m);
   uint32_t pk[2][32];
   float2 la = make_float2(0.f, 0.f), lb = make_float2(0.f, 0.f);
@@ -816,7 +821,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       const float sl2 = p.scale_log2;
       const int tail_valid = p.Sk - (n_kv_total - 1) * kTileN;  // 1..128 valid keys in the last tile of K
-      float m_used = -INFINITY;
+      float m_used = -INFINITY, neg_m = 0.f;
       float l_sum = 0.f;
 
       int jt = rot;  // the CTA's tile of step j (advanced without a division)
@@ -825,7 +830,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int j = 0; j < n_kv; ++j) {
         mbar_wait(bar_s_full + 8 * t, j & 1, abort_flag, p.status, kDevTimeoutSoftmax);
         tc_fence_after_sync();
-        softmax_step<kFp16>(t_s, t_o, bar_p_full + 16 * t, j == 0, jt == last_rel ? tail_valid : kTileN, sl2, m_used, l_sum);
+        softmax_step<kFp16>(t_s, t_o, bar_p_full + 16 * t, j == 0, jt == last_rel ? tail_valid : kTileN, sl2, m_used, neg_m, l_sum);
         if (++jt == n_kv) jt = 0;
       }
 
