@@ -124,9 +124,6 @@ struct AttnParams {
   const float2* q_table;  // (cos, sin) pairs, [rows][64]
   int q_table_rows, q_gf, q_gh, q_gw, q_n_t, q_n_h;
   long long q_pos_offset;
-#ifdef CHITU_ATTN_TIMING
-  long long* dbg;   // per-phase clock totals of CTA 0 (development builds only)
-#endif
 };
 
 template <bool kFp16>
@@ -455,18 +452,6 @@ __device__ __forceinline__ void push_rows(const AttnParams& p, int id, int n) {
   }
 }
 
-#ifdef CHITU_ATTN_TIMING
-#define CHITU_TRACE(i)                                                                                       \
-  do {                                                                                                       \
-    if (p.dbg != nullptr) {                                                                                  \
-      unsigned long long t_;                                                                                 \
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));                                                 \
-      p.dbg[64 + 8 * (blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) + (i)] = (long long)t_; \
-    }                                                                                                        \
-  } while (0)
-#else
-#define CHITU_TRACE(i)
-#endif
 
 // Thread-block cluster helpers (cluster_merge).
 __device__ __forceinline__ void cluster_sync_all() {
@@ -520,10 +505,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  if (threadIdx.x == 0) CHITU_TRACE(0);
   if (p.push_ctas > 0 && static_cast<int>(blockIdx.x) < p.push_ctas) {  // a copy CTA: no tensor memory, no barriers
     push_rows(p, blockIdx.x, p.push_ctas);
-    if (threadIdx.x == 0) CHITU_TRACE(6);
     return;
   }
   int bx, by, bz;
@@ -630,14 +613,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if ((ready >> src) & 1u) continue;
         if (!wait_flag(flags + src, flag_epoch, p.flag_timeout, p.status)) *abort_flag = 1;
         ready |= 1u << src;
-        CHITU_TRACE(1);
         // the rows were written by a peer's ordinary stores and are about to be read by the copy engine
         asm volatile("fence.proxy.async.global;" ::: "memory");
       }
     };
     if (lane == 0) {
       wait_rows(p.push_ctas > 0 ? p.q_flags : p.in_flags, q_ready, q0, q0 + n_qt * kTileM, p.Sq);
-      CHITU_TRACE(7);
       for (int t = 0; t < n_qt; ++t) {
         mbar_arrive_expect_tx(bar_q_full + 8 * t, kTileBytes);
         tma_load_4d(q_smem + t * kTileBytes, &tm_q, bar_q_full + 8 * t, 0, head, q0 + t * kTileM, batch);
@@ -663,7 +644,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       __syncwarp();
     }
-    if (lane == 0) CHITU_TRACE(2);
     if (*abort_flag && lane == 0) {
       // A role gave up: make sure no bulk copy of ours is still landing in this
       // CTA's shared memory before the CTA retires (bounded polls): the Q tiles, then the last
@@ -796,28 +776,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint32_t t_o = tmem_base + lane_base + 2 * kTileN + t * kHeadDim;
       if (q_fuse) {
         // this tile's four warps: fetch rotary factors, wait for the tile, rewrite it, hand it to the MMA warp
-#ifdef CHITU_ATTN_TIMING
-        long long qt0 = clock64(), qt1 = 0;
-#endif
         transform_q_tile<kFp16>(smem_gen + t * kTileBytes, quad, lane, head, batch, q0 + t * kTileM, p, [&] {
-#ifdef CHITU_ATTN_TIMING
-          qt1 = clock64();
-#endif
           mbar_wait(bar_q_full + 8 * t, 0, abort_flag, p.status, kDevTimeoutSoftmax);
-#ifdef CHITU_ATTN_TIMING
-          if (p.dbg != nullptr && bx == 0 && by == 0 && bz == 0 && threadIdx.x == 0) {
-            p.dbg[24] = qt1 - qt0;
-            p.dbg[25] = clock64() - qt1;
-            qt1 = clock64();
-          }
-#endif
         });
         fence_proxy_async_smem();  // the rewritten tile is read by the tensor core through the async proxy
         mbar_arrive(bar_q_ready + 8 * t);
-#ifdef CHITU_ATTN_TIMING
-        if (p.dbg != nullptr && bx == 0 && by == 0 && bz == 0 && threadIdx.x == 0)
-          p.dbg[26] = clock64() - qt1;
-#endif
       }
       const float sl2 = p.scale_log2;
       const int tail_valid = p.Sk - (n_kv_total - 1) * kTileN;  // 1..128 valid keys in the last tile of K
@@ -835,7 +798,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
 
       // epilogue: O / l -> 16-bit, row-contiguous 256-byte stores; LSE in natural log
-      if (t == 0 && row_in_tile == 0) CHITU_TRACE(3);
       mbar_wait(bar_o_final + 8 * t, 0, abort_flag, p.status, kDevTimeoutEpilogue);
       tc_fence_after_sync();
       int qblock, head, ez;
@@ -1034,7 +996,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
       }
-      if (t == 0 && row_in_tile == 0) CHITU_TRACE(4);
       if (write_out && p.lse != nullptr && row < p.Sq)
         p.lse[(static_cast<size_t>(batch) * p.H + head) * p.Sq + row] = lse_row;
     }
@@ -1042,14 +1003,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   tc_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x == 0) CHITU_TRACE(5);
   if (warp == 8) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
   if (p.signal_out && threadIdx.x == 0)
     publish_when_last(p.sync, kSyncAttnDone, kSyncOutEpoch, kSyncOutFlag, p.push_ctas > 0 ? p.grid_q * p.grid_h * p.grid_z : gridDim.x * gridDim.y * gridDim.z);
-  if (threadIdx.x == 0) CHITU_TRACE(6);
 }
 
 }  // namespace chitu

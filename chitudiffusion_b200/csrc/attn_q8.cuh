@@ -41,9 +41,6 @@ struct AttnQ8Params {
   const float* k_scale;   // [B, H, ceil(Sk / 64)]
   const unsigned* v_amax; // [B, H, 128] bit patterns of max |v| per channel (dequantisation = amax / 448)
   const float* q_corr;    // [B, H, Sq] q' . mean(k) in the base-2 domain (undoes the K centring in the LSE)
-#ifdef CHITU_ATTN_TIMING
-  long long* dbg;
-#endif
 };
 
 // 2^x for a pair of values on the FMA pipe, quadratic form of exp2_poly2 (max relative error 1.7e-3:

@@ -129,10 +129,6 @@ int g_cluster_merge = 1;
 
 }  // namespace
 
-#ifdef CHITU_ATTN_TIMING
-static long long* g_dbg = nullptr;
-extern "C" void chitu_b200_set_dbg(long long* ptr) { g_dbg = ptr; }
-#endif
 
 extern "C" {
 
@@ -547,9 +543,6 @@ int attn_fwd_impl(const void* q, const void* k, const void* v, void* out, const 
     // the rank, so that the receivers do not all ask the same source first
     p.rot_other = static_cast<int>((static_cast<long long>(me % len) * ex.rows_per_src) / chitu::kTileN);
   }
-#ifdef CHITU_ATTN_TIMING
-  p.dbg = g_dbg;
-#endif
 
   static bool attr_done[2][kMaxDevices] = {};
   static std::mutex attr_mu;
@@ -1166,10 +1159,11 @@ int chitu_b200_layernorm_modulate(const void* x, int x_dtype, void* out, int out
     const int64_t resident = std::max<int64_t>(1, 148 * per_sm / batches);
     const dim3 grid(static_cast<unsigned>(std::min<int64_t>(groups, resident)), static_cast<unsigned>(batches));
 #define CHITU_LN(DT) \
-    (two              ? chitu::layernorm_affine_rows_kernel<DT, 2, 1024><<<grid, threads, 0, st>>>(p) \
-     : threads <= 384 ? chitu::layernorm_affine_rows_kernel<DT, 1, 384><<<grid, threads, 0, st>>>(p) \
-                      : chitu::layernorm_affine_rows_kernel<DT, 1, 1024><<<grid, threads, 0, st>>>(p))
-    if (x_dtype == CHITU_DTYPE_BF16)
+    (threads <= 384 ? chitu::layernorm_affine_rows_kernel<DT, 1, 384><<<grid, threads, 0, st>>>(p) \
+                    : chitu::layernorm_affine_rows_kernel<DT, 1, 1024><<<grid, threads, 0, st>>>(p))
+    if (two)  // (16-bit rows end at 1024 vectors)
+      chitu::layernorm_affine_rows_kernel<2, 2, 1024><<<grid, threads, 0, st>>>(p);
+    else if (x_dtype == CHITU_DTYPE_BF16)
       CHITU_LN(0);
     else if (x_dtype == CHITU_DTYPE_FP16)
       CHITU_LN(1);
@@ -1521,9 +1515,6 @@ extern "C" int chitu_b200_attn_fwd_q8(const void* q, const void* k, const void* 
   p.k_scale = k_scale;
   p.v_amax = v_amax;
   p.q_corr = q_corr;
-#ifdef CHITU_ATTN_TIMING
-  p.dbg = g_dbg;
-#endif
   static bool attr_done[2][kMaxDevices] = {};
   static std::mutex attr_mu;
   const cudaError_t attr_err =
