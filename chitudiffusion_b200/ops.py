@@ -44,8 +44,15 @@ def _launched(n: int = 1) -> None:
     launch_count += n
 
 
+# the devices that tensors carry (a look-up costs a third of asking the object for its type and index)
+_CUDA_INDEX = {torch.device("cuda", i): i for i in range(64)}
+
+
 def _device_key(device) -> int:
     """Index of a device given in any of the forms torch takes: an object, a name, an index, None for the current one."""
+    index = _CUDA_INDEX.get(device)
+    if index is not None:
+        return index
     if not isinstance(device, torch.device):
         device = torch.device("cuda" if device is None else device)
     if device.type != "cuda":
@@ -55,7 +62,8 @@ def _device_key(device) -> int:
 
 def _stream_ptr(device) -> int:
     # the handle alone: building a torch Stream object costs ten times as much and every call needs it
-    return torch._C._cuda_getCurrentRawStream(_device_key(device))
+    index = _CUDA_INDEX.get(device)
+    return torch._C._cuda_getCurrentRawStream(_device_key(device) if index is None else index)
 
 
 class _NoGuard:
@@ -71,9 +79,9 @@ _NO_GUARD = _NoGuard()
 
 def _on(device):
     """``torch.cuda.device(device)`` where that changes anything (entering and leaving it costs some microseconds)."""
-    if isinstance(device, torch.device) and device.type == "cuda":
-        if device.index is None or torch._C._cuda_getDevice() == device.index:
-            return _NO_GUARD
+    index = _CUDA_INDEX.get(device)
+    if index is not None and torch._C._cuda_getDevice() == index:
+        return _NO_GUARD
     return torch.cuda.device(device)
 
 

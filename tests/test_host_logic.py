@@ -82,9 +82,9 @@ def test_devices_in_every_form_that_torch_takes(monkeypatch):
         with ops._on(device):
             pass
     # a guard is entered for another device than the current one, and for the forms that only torch itself resolves
-    assert entered == [torch.device("cuda", 1), "cuda:2", "cuda", 0, None]
+    assert entered == [torch.device("cuda", 1), torch.device("cuda"), "cuda:2", "cuda", 0, None]
     with ops._on(torch.device("cuda", 3)):
-        assert len(entered) == 5
+        assert len(entered) == 6
     ops._on(torch.device("cpu"))  # left to torch, which refuses it
     assert entered[-1] == torch.device("cpu")
     with pytest.raises(ValueError, match="cuda device"):
