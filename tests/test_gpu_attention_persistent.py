@@ -166,3 +166,47 @@ def test_a_cut_that_does_not_pay_is_not_taken():
     assert _need(1, 2560, 2048, 24) == 0  # 240 x 16: 64, 67
     assert _need(1, 4608, 4608, 24) == 0  # 432 x 36: 202, 213
     assert _need(1, 2560, 8192, 15) > 0  # 150 x 64: 209, 140
+
+
+def test_two_streams_cut_at_once():
+    from chitudiffusion_b200 import ops
+
+    sets = [[t.cuda() for t in _inputs(1, 1100, 1500, 37, torch.bfloat16, seed)] for seed in (11, 12)]
+    want = [ops.attn_fwd(*s)[0] for s in sets]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in sets]
+    outs = [[], []]
+    for _ in range(8):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                outs[i].append(ops.attn_fwd(*sets[i])[0])
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(o, want[i]) for o in outs[i])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("H,n_splits", [(40, None), (2, 3)])
+def test_the_first_call_of_a_process_may_be_a_captured_one(H, n_splits):
+    """Status word and scratch come into being inside the capture; a child process, so that this is its first call."""
+    import os
+    import subprocess
+    import sys
+
+    code = f"""
+import torch
+from chitudiffusion_b200 import ops
+q, k, v = (torch.randn(1, s, {H}, 128, device="cuda").bfloat16() for s in (1100, 1500, 1500))
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    out, _ = ops.attn_fwd(q, k, v, n_splits={n_splits})
+graph.replay()
+torch.cuda.synchronize()
+ref, _ = ops.attn_fwd(q, k, v, n_splits=1)
+assert (out.float() - ref.float()).abs().max().item() <= 2 ** -7 * ref.float().abs().max().item()
+ops.check_status()
+"""
+    root = os.path.abspath(os.path.join(os.path.dirname(__file__), ".."))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
