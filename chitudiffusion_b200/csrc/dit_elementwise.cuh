@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256) layernorm_affine_warp_kernel(const LayerN
 // fp32 (cold L2, 6 us of launch and event included): 24.6, 31.6, 65.5, 33.8 with a warp (5120: a block) per row, so
 // 18.5, 24.6, 65.4, 22.6.
 // Up to 384 threads run two (fp32, whose rows hold half as many channels per thread: three) CTAs per SM, wider rows
-// with 64 registers and half as many rows in flight.
+// with 64 registers and half as many rows in flight (two CTAs up to 512 threads).
 template <int kXDtype, int kVec, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, kMaxThreads > 384 ? 1 : kXDtype == 2 ? 3 : 2) layernorm_affine_rows_kernel(const LayerNormParams p) {
   constexpr int kLnRows = kMaxThreads <= 384 ? 4 : 2;
@@ -408,8 +408,8 @@ gate_residual_kernel(const GateResidualParams p) {
 // Column form of the same update: a thread owns eight channels (its gate sits in registers) of every row its CTA
 // visits, four rows in flight.  The CTA's threads are rows_par rows side by side, blockIdx.y is the batch.  (The
 // general kernel divides 64-bit indices for every 4 elements and reads the gate each time.)  HBM bound; us at
-// 4096 / 6889 x 3072 bf16 and 32760 x 1536 fp32 (cold L2, 6 us of launch and event included): 35.7, 55.3, 109.5 ->
-// 20.5, 28.7, 86.1.
+// 4096 x 3072 bf16, 1024 x 3072 and 32760 x 1536 fp32 (inputs larger than L2, launches in a graph): 31.2, 8.4, 104.6 ->
+// 14.3, 8.3, 80.5 (5.3, 4.5 and 6.2 TB/s).
 template <int kXDtype, bool kYFp16, int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads) gate_residual_rows_kernel(const GateResidualParams p, int rows_par) {
   constexpr int kGateRows = kMaxThreads <= 512 ? 4 : 2;

@@ -89,7 +89,7 @@ int chitu_b200_attn_fwd_splitkv(const void* q, const void* k, const void* v, voi
 /*
  * chitu_b200_attn_fwd with a workspace that lets the call finish evenly on all SMs: 256-row query blocks run one
  * per SM, and the ones left over for a last, partly filled wave are cut along the keys into equal pieces, one per
- * SM; the CTA that completes a query block's last piece merges its fp32 partial rows from the workspace.  Whether
+ * SM; the warp that completes the last piece of its 32 rows merges their fp32 partials from the workspace.  Whether
  * a call is cut is decided from its sizes; chitu_b200_attn_balanced_workspace_bytes returns the scratch that it then
  * needs (at most about 40 MB; 0: nothing is cut) on the current device.  A NULL workspace runs whole query blocks.
  * Workspace rules as for chitu_b200_attn_fwd_splitkv (16-byte aligned, zero header, one call at a time), and
