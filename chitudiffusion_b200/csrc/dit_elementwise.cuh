@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads > 384 ? 1 : kXDtype =
         for (int e = 0; e < kPer; ++e) s[r] += f[e];
       }
     }
-    block_sums<kLnRows>(s, red[0], n_warps);
+    block_sums<kLnRows, kLnRows == 4 || kVec == 2>(s, red[0], n_warps);
 #pragma unroll
     for (int r = 0; r < kLnRows; ++r) {
       mean[r] = s[r] * inv_c;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads > 384 ? 1 : kXDtype =
         for (int e = 0; e < kPer; ++e) s[r] = fmaf(f[e] - mean[r], f[e] - mean[r], s[r]);
       }
     }
-    block_sums<kLnRows>(s, red[1], n_warps);
+    block_sums<kLnRows, kLnRows == 4 || kVec == 2>(s, red[1], n_warps);
 #pragma unroll
     for (int r = 0; r < kLnRows; ++r) {
       const float rstd = rsqrtf(s[r] * inv_c + p.eps);

@@ -61,34 +61,55 @@ __device__ __forceinline__ void st4(void* p, int dtype, size_t i, float4 v) {
 }
 
 // Sums of kRows values (2 or 4) over the block, in every thread; one barrier.  red[kRows][32] must not be in use by an
-// earlier call that a thread of the block may still be in (two buffers in turn are enough).  The rows are folded into
-// each other on the way through the warp - 13 shuffles for four rows instead of 40.
-template <int kRows>
+// earlier call that a thread of the block may still be in (two buffers in turn are enough).
+//
+// kFold: the rows are folded into each other on the way through the warp - 13 shuffles for four rows instead of 40, 11
+// for two instead of 20, but in one chain where two rows have two side by side.  Four rows always fold; two rows
+// where the threads have registers to spare do not (us, folded / not: norm + rotary of 4100 x 3072 fp32 34.9 / 29.8, LayerNorm of
+// 8192 x 2560 fp32 35.1 / 28.4), and do at the 64 registers of wide rows (norm + rotary of 4100 x 5120 fp32 67.8 / 80.8,
+// LayerNorm of 8192 x 5120 fp32, two vectors a thread, 55.8 / 62.9).
+template <int kRows, bool kFold>
 __device__ __forceinline__ void block_sums(float (&s)[kRows], float (*red)[32], int n_warps) {
   static_assert(kRows == 2 || kRows == 4, "rows that fold into a warp");
-  constexpr int kGroup = 32 / kRows;  // lanes per row once folded
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool hi = lane & 16;
-  float v;
-  if constexpr (kRows == 4) {
-    const float a = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16);
-    const float b = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
-    const bool odd = lane & 8;
-    v = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+  if constexpr (kFold) {
+    constexpr int kGroup = 32 / kRows;  // lanes per row once folded
+    const bool hi = lane & 16;
+    float v;
+    if constexpr (kRows == 4) {
+      const float a = (hi ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[2], 16);
+      const float b = (hi ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, hi ? s[1] : s[3], 16);
+      const bool odd = lane & 8;
+      v = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+    } else {
+      v = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 16);
+    }
+#pragma unroll
+    for (int o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int row = lane / kGroup, l = lane % kGroup;
+    if (l == 0) red[row][warp] = v;
+    __syncthreads();
+    v = 0.f;
+    for (int w = l; w < n_warps; w += kGroup) v += red[row][w];
+#pragma unroll
+    for (int o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) s[r] = __shfl_sync(0xffffffffu, v, r * kGroup);
   } else {
-    v = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], 16);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+      if (lane == 0) red[r][warp] = s[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      s[r] = lane < n_warps ? red[r][lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+    }
   }
-#pragma unroll
-  for (int o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int row = lane / kGroup, l = lane % kGroup;
-  if (l == 0) red[row][warp] = v;
-  __syncthreads();
-  v = 0.f;
-  for (int w = l; w < n_warps; w += kGroup) v += red[row][w];
-#pragma unroll
-  for (int o = kGroup / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) s[r] = __shfl_sync(0xffffffffu, v, r * kGroup);
 }
 
 // ----------------------------------------------------------------------------
@@ -305,8 +326,9 @@ struct NormRopeTokens {
 // One job of a launch.  Everything that does not change inside a launch is a template argument, so
 // the token loop carries no run-time mode tests: kNormMode / kRopeMode as documented at
 // NormRopeParams, kRound 0 (no intermediate rounding), 1 (round the normalised value to the input
-// type, as `type_as(x)` does) or 2 (also round after the weight multiply), kOutBf16 the store type.
-template <int kInDtype, int kNormMode, int kRopeMode, int kRound, bool kOutBf16>
+// type, as `type_as(x)` does) or 2 (also round after the weight multiply), kOutBf16 the store type, kWide the entry
+// point for wide rows.
+template <int kInDtype, int kNormMode, int kRopeMode, int kRound, bool kOutBf16, bool kWide>
 __device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float (*red)[NormRopeTokens<kInDtype>::value][32]) {
   constexpr int kTok = NormRopeTokens<kInDtype>::value;
   constexpr int kOutDtype = kOutBf16 ? kBF16 : kFP16;
@@ -368,7 +390,7 @@ __device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float 
         for (int e = 0; e < 8; ++e) ss = fmaf(v[e], v[e], ss);
         rstd_full[i] = ss;
       }
-      block_sums<kTok>(rstd_full, red[phase], n_warps);  // red[phase] is rewritten two iterations later
+      block_sums<kTok, kTok == 4 || kWide>(rstd_full, red[phase], n_warps);  // red[phase] is rewritten two iterations later
 #pragma unroll
       for (int i = 0; i < kTok; ++i) rstd_full[i] = rsqrtf(rstd_full[i] * inv_n + p.eps);
     }
@@ -499,14 +521,14 @@ __device__ __forceinline__ void qk_norm_rope_job(const NormRopeParams& p, float 
 
 // Picks the instance of the job blockIdx.y points at: a job whose own modes are (2, 0) is a plain
 // cast / scatter whatever the launch's template modes are.
-template <int kInDtype, int kNormModeT, int kRopeModeT>
+template <int kInDtype, int kNormModeT, int kRopeModeT, bool kWide>
 __device__ __forceinline__ void qk_norm_rope_dispatch(const NormRopeBatch& batch,
                                                       float (*red)[NormRopeTokens<kInDtype>::value][32]) {
   const NormRopeParams& p = batch.job[blockIdx.y];
   const bool out_bf16 = p.out_dtype == kBF16;
   if (p.norm_mode == 2 && p.rope_mode == 0) {
-    if (out_bf16) qk_norm_rope_job<kInDtype, 2, 0, 0, true>(p, red);
-    else qk_norm_rope_job<kInDtype, 2, 0, 0, false>(p, red);
+    if (out_bf16) qk_norm_rope_job<kInDtype, 2, 0, 0, true, kWide>(p, red);
+    else qk_norm_rope_job<kInDtype, 2, 0, 0, false, kWide>(p, red);
     return;
   }
   // rounding of the weight product only where the reference's dtypes make it round (16-bit weight
@@ -515,23 +537,23 @@ __device__ __forceinline__ void qk_norm_rope_dispatch(const NormRopeBatch& batch
   const bool round_w = round_mid && p.weight != nullptr && p.w_dtype != kFP32 && kInDtype != kFP32;
   const int round = round_w ? 2 : (round_mid ? 1 : 0);
   if (out_bf16) {
-    if (round == 0) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 0, true>(p, red);
-    else if (round == 1) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 1, true>(p, red);
-    else qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 2, true>(p, red);
+    if (round == 0) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 0, true, kWide>(p, red);
+    else if (round == 1) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 1, true, kWide>(p, red);
+    else qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 2, true, kWide>(p, red);
   } else {
-    if (round == 0) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 0, false>(p, red);
-    else if (round == 1) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 1, false>(p, red);
-    else qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 2, false>(p, red);
+    if (round == 0) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 0, false, kWide>(p, red);
+    else if (round == 1) qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 1, false, kWide>(p, red);
+    else qk_norm_rope_job<kInDtype, kNormModeT, kRopeModeT, 2, false, kWide>(p, red);
   }
 }
 
 // Picks the instance of the job blockIdx.y points at: a job whose own modes are (2, 0) is a plain
 // cast / scatter whatever the launch's template modes are.  A launch that feeds the fused exchange
 // ends by publishing "my rows have landed" to every peer (last-block pattern).
-template <int kInDtype, int kNormModeT, int kRopeModeT>
+template <int kInDtype, int kNormModeT, int kRopeModeT, bool kWide>
 __device__ __forceinline__ void qk_norm_rope_body(const NormRopeBatch& batch) {
   __shared__ float red[2][NormRopeTokens<kInDtype>::value][32];
-  qk_norm_rope_dispatch<kInDtype, kNormModeT, kRopeModeT>(batch, red);
+  qk_norm_rope_dispatch<kInDtype, kNormModeT, kRopeModeT, kWide>(batch, red);
   if (batch.signal) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -549,12 +571,12 @@ __device__ __forceinline__ void qk_norm_rope_body(const NormRopeBatch& batch) {
 // CTAs of 384 threads per SM; wider rows run with the 64 registers that 1024 threads leave.
 template <int kInDtype, int kNormModeT, int kRopeModeT>
 __global__ void __maxnreg__(80) qk_norm_rope_kernel(const __grid_constant__ NormRopeBatch batch) {
-  qk_norm_rope_body<kInDtype, kNormModeT, kRopeModeT>(batch);
+  qk_norm_rope_body<kInDtype, kNormModeT, kRopeModeT, false>(batch);
 }
 template <int kInDtype, int kNormModeT, int kRopeModeT>
 __global__ void __launch_bounds__(kNormMaxThreads)
 qk_norm_rope_wide_kernel(const __grid_constant__ NormRopeBatch batch) {
-  qk_norm_rope_body<kInDtype, kNormModeT, kRopeModeT>(batch);
+  qk_norm_rope_body<kInDtype, kNormModeT, kRopeModeT, true>(batch);
 }
 
 // ----------------------------------------------------------------------------
