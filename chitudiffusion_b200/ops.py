@@ -165,7 +165,9 @@ def auto_key_splits(B: int, Sq: int, Sk: int, H: int) -> int:
     waves of one CTA per SM, so the cost of a call is (waves) x (key tiles per CTA, plus about 5 tile steps for
     a CTA's prologue and for parking its partial rows: 216 CTAs x 36 tiles measured 138 us, 432 CTAs x 18 tiles
     143 us) plus about one tile step per range for the merge.  The split that minimises it is taken when it
-    saves at least 8 %: it fills small grids (54 CTAs -> 2 ranges).
+    saves at least 8 %: it fills small grids (54 CTAs -> 2 ranges).  The model is that of ``attn_fwd_kernel``: it knows neither
+    the persistent kernel of plain calls above one wave nor the cut of its last wave, and still splits some grids
+    of 149 to about 220 blocks that the cut would serve better (150 x 60 tiles: two ranges 176 us, cut 135).
     ``CHITU_B200_KEY_SPLITS`` overrides."""
     forced = os.environ.get("CHITU_B200_KEY_SPLITS")
     tiles = -(-Sk // 128)
